@@ -21,7 +21,7 @@ namespace mvmcb {
 
 int launch_sample(const DevModel& m, const DevWalkers& w, int precision, cudaStream_t stream);
 bool sample_planes_in_smem(const DevModel& m, int precision, int limit);
-int launch_measure(const DevModel& m, const int* s_idx, const int* s_cfg, const int* s_num,
+int launch_measure(const DevModel& m, const MeasTables& mt, const int* s_idx, const int* s_cfg, const int* s_num,
                    const int* s_cnt, int nsamples, double* gws, int gws_blocks, double* ostore,
                    double* eloc, double* lpsi, int* valid, double* gval, unsigned* status, cudaStream_t stream);
 int launch_green_reduce(const DevModel& m, int W, int S, int n_one, int nex, const int* ex, const double* gval,
@@ -115,6 +115,7 @@ struct mvmc_b200_ctx {
   cudaStream_t stream = nullptr;
   DevModel dm{};
   DevWalkers dw{};
+  MeasTables mt{};
   std::vector<void*> allocs;
   double* d_f = nullptr;
   double* d_proj = nullptr;
@@ -407,7 +408,10 @@ void build_context(mvmc_b200_ctx* c, const char* namelist, const char* initial_d
   dm.trans = c->upload(trans);
   dm.trans_sgn = c->upload(trans_sgn);
   dm.spgl = c->upload(spgl);
-  // Slater-derivative site pairs by orbital (deterministic O_k of the packed measurement)
+  // Slater-derivative site pairs by orbital (the deterministic O_k)
+  MeasTables& mt = c->mt;
+  std::vector<int2> at;
+  std::vector<int> folded;
   {
     std::vector<std::vector<int>> by_orb(std::max(0, m.n_orb));
     for (int a = 0; a < ns; ++a)
@@ -436,6 +440,52 @@ void build_context(mvmc_b200_ctx* c, const char* namelist, const char* initial_d
       dm.orb_off = c->upload(off);
       dm.orb_ent = c->upload(ent);
       dm.trans_inv = c->upload(tinv);
+      // the same pairs per translation, signs folded in; interleaved over the orbitals unless
+      // padding to the longest list would more than double the table
+      size_t longest = 0;
+      for (const auto& v : by_orb) longest = std::max(longest, v.size());
+      const bool even = longest * by_orb.size() <= 2 * ent.size();
+      mt.orb_stride = even ? static_cast<int>(by_orb.size()) : 1;
+      mt.orb_len = even ? longest * by_orb.size() : ent.size();
+      folded.assign(static_cast<size_t>(dm.nmp) * mt.orb_len, 0);
+      at.resize(by_orb.size());
+      for (size_t k = 0; k < by_orb.size(); ++k) {
+        at[k] = make_int2(even ? static_cast<int>(k) : off[k], static_cast<int>(by_orb[k].size()));
+        for (int mp = 0; mp < dm.nmp; ++mp)
+          for (size_t e = 0; e < by_orb[k].size(); ++e) {
+            const int v = by_orb[k][e];
+            const int a = tinv[mp * ns + (v >> 16)], b = tinv[mp * ns + ((v >> 1) & 0x7fff)];
+            const int sign = ((v & 1) ? -1 : 1) * trans_sgn[mp * ns + a] * trans_sgn[mp * ns + b];
+            folded[mp * mt.orb_len + at[k].x + e * mt.orb_stride] = (a << 16) | (b << 1) | (sign < 0 ? 1 : 0);
+          }
+      }
+    }
+  }
+  {
+    std::vector<std::vector<int2>> by_dst(ns2);
+    for (size_t t = 0; t < tval.size(); ++t) {
+      const int* h = &tterm[4 * t];
+      if (h[1] == h[3] && h[0] != h[2])
+        by_dst[h[0] + h[1] * ns].push_back(make_int2(h[2] + h[3] * ns, static_cast<int>(t)));
+    }
+    std::vector<int> hop_off(1, 0);
+    std::vector<int2> hop;
+    for (const auto& v : by_dst) {
+      hop.insert(hop.end(), v.begin(), v.end());
+      hop_off.push_back(static_cast<int>(hop.size()));
+    }
+    // one upload for the four tables, the pairs first (8-byte aligned)
+    std::vector<int> all;
+    for (const std::vector<int2>* v : {&hop, &at})
+      for (const int2& p : *v) all.insert(all.end(), {p.x, p.y});
+    all.insert(all.end(), hop_off.begin(), hop_off.end());
+    all.insert(all.end(), folded.begin(), folded.end());
+    const int* base = c->upload(all);
+    mt.hop = reinterpret_cast<const int2*>(base);
+    mt.hop_off = base + 2 * (hop.size() + at.size());
+    if (!folded.empty()) {
+      mt.orb_at = mt.hop + hop.size();
+      mt.orb_ent = mt.hop_off + hop_off.size();
     }
   }
   dm.tterm = c->upload(tterm);
@@ -560,7 +610,7 @@ int do_measure(mvmc_b200_ctx* c) {
     if (rc != kOk) return rc;
     rc = launch_reduce_totals(c->dm, c->W, c->d_wsum, c->d_tot, c->stream);
   } else {
-    rc = launch_measure(c->dm, c->dw.s_idx, c->dw.s_cfg, c->dw.s_num, c->dw.s_cnt, rows, c->d_gws, c->gws_blocks,
+    rc = launch_measure(c->dm, c->mt, c->dw.s_idx, c->dw.s_cfg, c->dw.s_num, c->dw.s_cnt, rows, c->d_gws, c->gws_blocks,
                         c->d_ostore, c->d_eloc, c->d_lpsi, c->d_valid, nullptr, c->dw.status, c->stream);
     if (rc != kOk) return rc;
     rc = launch_reduce(c->dm, c->W, c->S, c->d_ostore, c->d_eloc, c->d_valid, c->dw.s_num, c->d_wsum, c->d_tot,
@@ -590,7 +640,7 @@ int do_measure_green(mvmc_b200_ctx* c, std::vector<double>& gout) {
     c->d_gval = c->alloc<double>(need);
     c->gval_cap = need;
   }
-  int rc = launch_measure(c->dm, c->dw.s_idx, c->dw.s_cfg, c->dw.s_num, c->dw.s_cnt, static_cast<int>(rows), c->d_gws,
+  int rc = launch_measure(c->dm, c->mt, c->dw.s_idx, c->dw.s_cfg, c->dw.s_num, c->dw.s_cnt, static_cast<int>(rows), c->d_gws,
                           c->gws_blocks, nullptr, c->d_eloc, c->d_lpsi, c->d_valid, c->d_gval, c->dw.status,
                           c->stream);
   if (rc != kOk) return rc;

@@ -30,6 +30,7 @@
 #include "common.cuh"
 #include "engine.cuh"
 #include "pfinv.cuh"
+#include "skewtile.cuh"
 
 namespace mvmcb {
 
@@ -101,7 +102,8 @@ __device__ double hop_log_proj(const DevModel& m, int src, int dst, Occ occ) {
 // Σ_k α_k Δc_k of the hop src → dst (spin-site slots src_slot, dst_slot) from the
 // charges before the move and cj[r] = Σ_site J(r, site)·(n_site − 1): the O(1) form of
 // calh1_direct_projection_ratio_moved (observables.rs:1680-1758).
-__device__ inline double direct_hop_log_proj(const DevModel& m, const int* num, const double* cj, int source,
+template <class Num>
+__device__ inline double direct_hop_log_proj(const DevModel& m, const Num* num, const double* cj, int source,
                                              int dest, int src_slot, int dst_slot) {
   const int ns = m.ns;
   auto occ = [&](int slot) { return slot == src_slot ? 0 : (slot == dst_slot ? 1 : num[slot]); };
@@ -610,174 +612,147 @@ __global__ void __launch_bounds__(NT, (kSmemPlane || NT > kMeasThreads ? 1 : 2))
   }
 }
 
-// ---- planes whose strict upper triangle fits shared memory -----------------------------
-// For n where the full FP64 plane does not fit one SM (2D 16×16, n = 224: 401 KB) the
-// sample's plane is swept as a packed upper triangle in shared memory (gj_pfinv_packed,
-// 195 KB at n = 224), one 512-thread CTA per SM striding over the samples; nothing of the
-// sweep touches L2. The transfer terms' per-term sums sit in the block's L2 workspace. The
-// Slater derivative is gathered per orbital: thread k walks orbital k's translated site
-// pairs in a fixed order and adds the electron pairs on them, so O rows are bitwise
-// repeatable (no atomics).
-struct PackedLayout {
-  size_t idx, cfg, num, cnt, tr, tsg, pf, cj, rs, rowp, rowq, plane, total;
+// ---- O rows and energies with the planes as tiles of the upper triangle -----------------------
+// A sample's planes are swept one after the other as tiles in shared memory (skewtile.cuh):
+// nothing of the sweep leaves the SM, up to n = 224. NT threads per sample: 64 for n ≤ 64 and
+// many samples, so that several share an SM and hide each other's pivot chains, 512 for the
+// planes that fill an SM. The transfer terms run by destination (one Slater row is gathered for all
+// electrons that may hop there), the Slater derivative per orbital: thread k adds the electron
+// pairs on orbital k's site pairs in a fixed order, so O rows are bitwise repeatable.
+// Small integers (sites, occupations) are kept as 16 and 8 bits: the n = 224 tiles leave 9 KB.
+struct TriLayout {
+  size_t idx, cfg, num, cnt, pf, cj, acc, pan, tiles, total;
 };
 
-__host__ __device__ inline PackedLayout packed_layout(const DevModel& m) {
-  PackedLayout L;
+__host__ __device__ inline TriLayout tri_layout(const DevModel& m, bool acc_smem) {
+  TriLayout L;
   size_t o = 0;
-  L.idx = o; o = a16(o + sizeof(int) * m.n);
-  L.cfg = o; o = a16(o + sizeof(int) * m.ns2);
-  L.num = o; o = a16(o + sizeof(int) * m.ns2);
+  L.idx = o; o = a16(o + sizeof(short) * m.n);
+  L.cfg = o; o = a16(o + sizeof(short) * m.ns2);
+  L.num = o; o = a16(o + m.ns2);
   L.cnt = o; o = a16(o + sizeof(int) * (m.nproj + 1));
-  L.tr = o; o = a16(o + sizeof(int) * m.ns);
-  L.tsg = o; o = a16(o + sizeof(int) * m.ns);
   L.pf = o; o = a16(o + sizeof(double) * (m.nqp + 2));
   L.cj = o; o = a16(o + sizeof(double) * m.ns);
-  L.rs = o; o = a16(o + sizeof(int) * m.n);
-  L.rowp = o; o = a16(o + 2 * sizeof(double) * m.n);
-  L.rowq = o; o = a16(o + sizeof(double) * m.n);
-  L.plane = o; o = a16(o + sizeof(double) * static_cast<size_t>(m.n) * (m.n - 1) / 2);
+  // plane sums of the transfer terms and of the orbitals (else the block's workspace and the
+  // O row itself)
+  L.acc = o; if (acc_smem) o = a16(o + sizeof(double) * (static_cast<size_t>(m.nterm) + m.norb));
+  L.pan = o; o = a16(o + sizeof(double) * tri_pan_doubles(m.n) + kTriRedBytes);
+  L.tiles = o; o += sizeof(double) * tri_tile_doubles(m.n);
   L.total = o;
   return L;
 }
 
-constexpr int kPackedThreads = 512;
-
-template <int JPL>
-__global__ void __launch_bounds__(kPackedThreads, 1)
-    k_measure_packed(DevModel m, const int* __restrict__ s_idx, const int* __restrict__ s_cfg,
-                     const int* __restrict__ s_num, const int* __restrict__ s_cnt, int nsamples,
-                     double* __restrict__ gws, size_t gws_stride, double* __restrict__ ostore,
-                     double* __restrict__ eloc, double* __restrict__ lpsi, int* __restrict__ valid, unsigned* status) {
+template <int NT, int PG, int CPT>
+__global__ void __launch_bounds__(NT)
+    k_measure_tri(DevModel m, MeasTables mt, const int* __restrict__ s_idx, const int* __restrict__ s_cfg,
+                  const int* __restrict__ s_num, const int* __restrict__ s_cnt, int nsamples, int acc_smem,
+                  double* __restrict__ gws, size_t gws_stride, double* __restrict__ ostore, double* __restrict__ eloc,
+                  double* __restrict__ lpsi, int* __restrict__ valid, unsigned* status) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const PackedLayout L = packed_layout(m);
-  int* idx = reinterpret_cast<int*>(smem + L.idx);
-  int* cfg = reinterpret_cast<int*>(smem + L.cfg);
-  int* num = reinterpret_cast<int*>(smem + L.num);
+  const TriLayout L = tri_layout(m, acc_smem != 0);
+  short* idx = reinterpret_cast<short*>(smem + L.idx);
+  short* cfg = reinterpret_cast<short*>(smem + L.cfg);
+  signed char* num = reinterpret_cast<signed char*>(smem + L.num);
   int* cnt = reinterpret_cast<int*>(smem + L.cnt);
-  int* tinv = reinterpret_cast<int*>(smem + L.tr);
-  int* tsg = reinterpret_cast<int*>(smem + L.tsg);
   double* pf = reinterpret_cast<double*>(smem + L.pf);
   double* cj = reinterpret_cast<double*>(smem + L.cj);
-  int* rs = reinterpret_cast<int*>(smem + L.rs);
-  double* rowp = reinterpret_cast<double*>(smem + L.rowp);
-  double* rowq = reinterpret_cast<double*>(smem + L.rowq);
-  double* P = reinterpret_cast<double*>(smem + L.plane);
-  const int n = m.n, ns = m.ns, ne = m.ne, tid = threadIdx.x, nt = blockDim.x;
-  const int lane = tid & 31, warp = tid >> 5, nwarp = nt >> 5;
-  double* tacc = gws + static_cast<size_t>(blockIdx.x) * gws_stride;  // [nterm] plane sums
-  double* g1 = tacc + m.nterm;                                          // [nterm] term values
-  __shared__ int s_bad;
-  for (int i = tid; i < n; i += nt) rs[i] = i * n - i * (i + 1) / 2 - i - 1;
+  double* pan = reinterpret_cast<double*>(smem + L.pan);
+  unsigned char* red = reinterpret_cast<unsigned char*>(pan + tri_pan_doubles(m.n));
+  double* T = reinterpret_cast<double*>(smem + L.tiles);
+  const int n = m.n, ns = m.ns, ne = m.ne, nb = tri_blocks(n);
+  const int tid = threadIdx.x, nt = NT, lane = tid & 31, warp = tid >> 5;
+  constexpr int nwarp = NT / 32;
+  constexpr int kLanes = (NT == 512 ? 224 : (PG == 128 ? 128 : 64)) / 32;  // columns per lane
+  double* tacc = acc_smem ? reinterpret_cast<double*>(smem + L.acc) : gws + static_cast<size_t>(blockIdx.x) * gws_stride;
+  __shared__ double s_part[2][nwarp];
 
   for (int sample = blockIdx.x; sample < nsamples; sample += gridDim.x) {
-    for (int k = tid; k < n; k += nt) idx[k] = s_idx[static_cast<size_t>(sample) * n + k];
+    double* orow = ostore + static_cast<size_t>(sample) * m.sr_size;
+    double* oacc = acc_smem ? tacc + m.nterm : orow + 1 + m.nproj;
+    bool any = false, any_pos = false;
+    for (int k = tid; k < n; k += nt) {
+      const int v = s_idx[static_cast<size_t>(sample) * n + k];
+      idx[k] = static_cast<short>(v);
+      any = any || v != 0;
+      any_pos = any_pos || v >= 0;
+    }
     for (int k = tid; k < m.ns2; k += nt) {
-      cfg[k] = s_cfg[static_cast<size_t>(sample) * m.ns2 + k];
-      num[k] = s_num[static_cast<size_t>(sample) * m.ns2 + k];
+      cfg[k] = static_cast<short>(s_cfg[static_cast<size_t>(sample) * m.ns2 + k]);
+      num[k] = static_cast<signed char>(s_num[static_cast<size_t>(sample) * m.ns2 + k]);
     }
     for (int k = tid; k < m.nproj; k += nt) cnt[k] = s_cnt[static_cast<size_t>(sample) * m.nproj + k];
     for (int k = tid; k < m.nterm; k += nt) tacc[k] = 0.0;
-    double* orow = ostore + static_cast<size_t>(sample) * m.sr_size;
-    for (int k = tid; k < m.norb; k += nt) orow[1 + m.nproj + k] = 0.0;
-    if (tid == 0) s_bad = 0;
-    __syncthreads();
-    for (int r = tid; r < ns; r += nt) {  // cj[r] = Σ_site J[r][site]·(n_site − 1)
+    for (int k = tid; k < m.norb; k += nt) oacc[k] = 0.0;
+    const bool bad_cfg = !(__syncthreads_or(any) && __syncthreads_or(any_pos));
+    bool singular = false;
+    for (int r = tid; r < ns; r += nt) {  // cj[r] = Σ_site J[r][site]·(n_site − 1), J symmetric
       double acc = 0.0;
+#pragma unroll 8
       for (int site = 0; site < ns; ++site)
-        acc += __ldg(m.jast_pair + r * ns + site) * static_cast<double>(num[site] + num[site + ns] - 1);
+        acc += __ldg(m.jast_pair + site * ns + r) * static_cast<double>(num[site] + num[site + ns] - 1);
       cj[r] = acc;
     }
-    if (tid == 0) {
-      bool all_zero = true, all_neg = true;
-      for (int k = 0; k < n; ++k) {
-        all_zero = all_zero && idx[k] == 0;
-        all_neg = all_neg && idx[k] < 0;
-      }
-      if (all_zero || all_neg) s_bad = 1;
-    }
-    __syncthreads();
-    if (s_bad) {
-      if (tid == 0) {
-        valid[sample] = 0;
-        eloc[sample] = 0.0;
-        lpsi[sample] = 0.0;
-      }
-      for (int k = tid; k < m.sr_size; k += nt) orow[k] = 0.0;
-      __syncthreads();
-      continue;
-    }
-    for (int q = 0; q < m.nqp; ++q) {
+    for (int q = 0; q < m.nqp && !bad_cfg; ++q) {
       double pfv;
-      int st;
+      int st = 0;
       if (m.rinv) {
-        // resident measurement: the upper triangle of the sampler's X⁻¹ of this sample
+        // resident measurement: the sampler's X⁻¹ of this sample
         const double* src = m.rinv + (static_cast<size_t>(sample) * m.nqp + q) * n * n;
-        for (int i = warp; i < n - 1; i += nwarp)
-          for (int j = i + 1 + lane; j < n; j += 32) P[rs[i] + j] = src[static_cast<size_t>(i) * n + j];
+        tri_fill(T, n, warp, nwarp, [&](int i, int j) { return src[static_cast<size_t>(i) * n + j]; });
         pfv = m.rpf[static_cast<size_t>(sample) * m.nqp + q];
-        st = 0;
         __syncthreads();
       } else {
-        for (int i = warp; i < n - 1; i += nwarp) {  // X(i, j), i < j, from the Slater table
-          const int ri = idx[i] + (i >= ne ? ns : 0);
-          const double* srow = m.slater + (static_cast<size_t>(q) * m.ns2 + ri) * m.ns2;
-          for (int j = i + 1 + lane; j < n; j += 32) P[rs[i] + j] = __ldg(srow + idx[j] + (j >= ne ? ns : 0));
-        }
-        __syncthreads();
-        gj_pfinv_packed<JPL, (kPackedThreads > 512 ? 1 : 2)>(P, rs, n, rowp, rowq, pfv, st);
+        const double* sl = m.slater + static_cast<size_t>(q) * m.ns2 * m.ns2;
+        tri_fill(T, n, warp, nwarp, [&](int i, int j) {
+          return __ldg(sl + static_cast<size_t>(idx[i] + (i >= ne ? ns : 0)) * m.ns2 + idx[j] + (j >= ne ? ns : 0));
+        });
+        tri_sweep<NT, PG, CPT>(T, pan, red, n, pfv, st);
       }
       if (st != 0) {
-        if (tid == 0) s_bad = 1;
-        __syncthreads();
+        singular = true;  // the same in every thread
         break;
       }
       if (tid == 0) pf[q] = pfv;
       const double wq = m.qpw[q];
-      // transfer terms: one-electron ratio on this plane (warp per term)
-      for (int t = warp; t < m.nterm; t += nwarp) {
-        const int ti = m.tterm[4 * t], tsi = m.tterm[4 * t + 1], tj = m.tterm[4 * t + 2], tsj = m.tterm[4 * t + 3];
-        const int dst = ti + tsi * ns, src = tj + tsj * ns;
-        if (tsi != tsj || (ti == tj) || num[dst] == 1 || num[src] == 0 || cfg[src] < 0) continue;
-        const int msj = cfg[src] + tsj * ne;
-        const int rsa = ti + tsj * ns;
-        const double* srow = m.slater + (static_cast<size_t>(q) * m.ns2 + rsa) * m.ns2;
-        double sv[JPL];  // the gathered Slater row: every load of the lane in flight at once
+      // transfer terms by destination: −Pf·Σ_k X⁻¹[m][k]·F(dst, k) for every electron m that
+      // may hop there (the moved electron's own entry meets X⁻¹[m][m] = 0)
+      for (int d = warp; d < m.ns2; d += nwarp) {
+        const int e0 = __ldg(mt.hop_off + d), e1 = __ldg(mt.hop_off + d + 1);
+        if (num[d] == 1 || e0 == e1) continue;
+        const double* srow = m.slater + (static_cast<size_t>(q) * m.ns2 + d) * m.ns2;
+        double sv[kLanes];
 #pragma unroll
-        for (int c = 0; c < JPL; ++c) {
+        for (int c = 0; c < kLanes; ++c) {
           const int k = lane + 32 * c;
-          sv[c] = k < n ? __ldg(srow + (k == msj ? ti : idx[k]) + (k >= ne ? ns : 0)) : 0.0;
+          sv[c] = k < n ? __ldg(srow + idx[k] + (k >= ne ? ns : 0)) : 0.0;
         }
-        double r = 0.0;
+        const int spin = d >= ns ? 1 : 0;
+        for (int e = e0; e < e1; ++e) {
+          const int2 h = __ldg(mt.hop + e);  // source slot, term
+          if (num[h.x] == 0 || cfg[h.x] < 0) continue;
+          const int mi = cfg[h.x] + spin * ne;
+          double r = 0.0;
 #pragma unroll
-        for (int c = 0; c < JPL; ++c) {
-          const int k = lane + 32 * c;
-          if (k < n) r += packed_at(P, rs, msj, k) * sv[c];
-        }
-        r = warp_sum(r);
-        if (lane == 0) {
-          const double v = wq * (-r * pfv);
-          if (q == 0) tacc[t] = v;  // a plain store: no read of the block's workspace
-          else tacc[t] += v;
+          for (int c = 0; c < kLanes; ++c) {
+            const int k = lane + 32 * c;
+            if (k < n) r += tri_get(T, nb, mi, k) * sv[c];
+          }
+          r = warp_sum(r);
+          if (lane == 0) tacc[h.y] += wq * (-r * pfv);
         }
       }
-      // Slater derivative by orbital: electron pairs (i, j) on the orbital's site pairs
+      // Slater derivative by orbital: electron pairs on its translated site pairs
       const int trans = q / m.nleg, spidx = q % m.nleg, mpidx = trans % m.nmp;
-      for (int k = tid; k < ns; k += nt) {
-        const int a = m.trans_inv[mpidx * ns + k];
-        tinv[k] = a;
-        tsg[a] = m.trans_sgn[mpidx * ns + a];
-      }
-      __syncthreads();
       const double cs = pfv * m.spgl[spidx], cc = pfv * m.spgl[m.nleg + spidx], ss = pfv * m.spgl[2 * m.nleg + spidx];
       const double fac[4] = {cs, -cc, ss, -cs};  // (up, up), (up, dn), (dn, up), (dn, dn)
+      const int* ents = mt.orb_ent + static_cast<size_t>(mpidx) * mt.orb_len;
       for (int k = tid; k < m.norb; k += nt) {
+        const int2 at = __ldg(mt.orb_at + k);  // first entry, count
         double acc = 0.0;
-        const int e1 = __ldg(m.orb_off + k + 1);
-        for (int e = __ldg(m.orb_off + k); e < e1; ++e) {
-          const int ent = __ldg(m.orb_ent + e);
-          const int a = tinv[ent >> 16], b = tinv[(ent >> 1) & 0x7fff];
-          const int sgn = (ent & 1 ? -1 : 1) * tsg[a] * tsg[b];
+        for (int e = 0; e < at.y; ++e) {
+          const int ent = __ldg(ents + at.x + static_cast<size_t>(e) * mt.orb_stride);
+          const int a = ent >> 16, b = (ent >> 1) & 0x7fff;
+          double pair = 0.0;
 #pragma unroll
           for (int sa = 0; sa < 2; ++sa) {
             const int ei = cfg[a + sa * ns];
@@ -786,21 +761,21 @@ __global__ void __launch_bounds__(kPackedThreads, 1)
             for (int sb = 0; sb < 2; ++sb) {
               const int ej = cfg[b + sb * ns];
               if (ej < 0) continue;
-              const double v = packed_at(P, rs, ei + sa * ne, ej + sb * ne);
-              acc += (fac[2 * sa + sb] * v) * static_cast<double>(sgn);
+              pair += fac[2 * sa + sb] * tri_get(T, nb, ei + sa * ne, ej + sb * ne);
             }
           }
+          acc += (ent & 1) ? -pair : pair;
         }
-        orow[1 + m.nproj + k] += wq * acc;
+        oacc[k] += wq * acc;
       }
       __syncthreads();
     }
-    if (s_bad) {
+    if (bad_cfg || singular) {
       if (tid == 0) {
         valid[sample] = 0;
         eloc[sample] = 0.0;
         lpsi[sample] = 0.0;
-        atomicOr(status, kDevSingular);
+        if (singular) atomicOr(status, kDevSingular);
       }
       for (int k = tid; k < m.sr_size; k += nt) orow[k] = 0.0;
       __syncthreads();
@@ -808,76 +783,97 @@ __global__ void __launch_bounds__(kPackedThreads, 1)
     }
     double ip = 0.0;
     for (int q = 0; q < m.nqp; ++q) ip += m.qpw[q] * pf[q];
+    // the local energy and the projection exponent in a fixed order: per thread over its
+    // terms, lanes by shuffles, warps in order
+    double en = 0.0, lp = 0.0;
     for (int t = tid; t < m.nterm; t += nt) {
-      const int ti = m.tterm[4 * t], tsi = m.tterm[4 * t + 1], tj = m.tterm[4 * t + 2], tsj = m.tterm[4 * t + 3];
+      const int4 h = __ldg(reinterpret_cast<const int4*>(m.tterm) + t);
+      const int ti = h.x, tsi = h.y, tj = h.z, tsj = h.w;
       const int dst = ti + tsi * ns, src = tj + tsj * ns;
       double g;
       if (tsi == tsj && ti == tj) g = static_cast<double>(num[src]);
       else if (tsi != tsj || num[dst] == 1 || num[src] == 0 || cfg[src] < 0) g = 0.0;
       else g = exp(direct_hop_log_proj(m, num, cj, tj, ti, src, dst)) * tacc[t] / ip;
-      // the transfer sum Σ_t −t_t·g_t in a fixed order: per thread over its terms, warps
-      // by shuffles, warps in order below
-      g1[t] = -m.tval[t] * g;
+      en -= m.tval[t] * g;
     }
-    double part = 0.0;
-    for (int t = tid; t < m.nterm; t += nt) part += g1[t];
-    part = warp_sum(part);
-    if (lane == 0) rowq[warp] = part;  // the sweep's row buffer is free here
+    for (int k = tid; k < m.nintra; k += nt) {
+      const int i = m.intra_i[k];
+      en += m.intra_v[k] * static_cast<double>(num[i] * num[i + ns]);
+    }
+    for (int k = tid; k < m.ninter; k += nt) {
+      const int i = m.inter_ij[2 * k], j = m.inter_ij[2 * k + 1];
+      en += m.inter_v[k] * static_cast<double>(num[i] + num[i + ns]) * static_cast<double>(num[j] + num[j + ns]);
+    }
+    for (int k = tid; k < m.nhund; k += nt) {
+      const int i = m.hund_ij[2 * k], j = m.hund_ij[2 * k + 1];
+      en -= m.hund_v[k] * (static_cast<double>(num[i] * num[j]) + static_cast<double>(num[i + ns] * num[j + ns]));
+    }
+    for (int k = tid; k < m.nproj; k += nt) lp += m.proj[k] * static_cast<double>(cnt[k]);
+    en = warp_sum(en);
+    lp = warp_sum(lp);
+    if (lane == 0) {
+      s_part[0][warp] = en;
+      s_part[1][warp] = lp;
+    }
     __syncthreads();
+    en = lp = 0.0;
+    for (int w = 0; w < nwarp; ++w) {
+      en += s_part[0][w];
+      lp += s_part[1][w];
+    }
+    const bool ok = fabs(ip) >= 1.0e-100 && isfinite(en);
     if (tid == 0) {
-      double e = 0.0;
-      for (int k = 0; k < m.nintra; ++k) {
-        const int i = m.intra_i[k];
-        e += m.intra_v[k] * static_cast<double>(num[i] * num[i + ns]);
-      }
-      for (int k = 0; k < m.ninter; ++k) {
-        const int i = m.inter_ij[2 * k], j = m.inter_ij[2 * k + 1];
-        e += m.inter_v[k] * static_cast<double>(num[i] + num[i + ns]) * static_cast<double>(num[j] + num[j + ns]);
-      }
-      for (int k = 0; k < m.nhund; ++k) {
-        const int i = m.hund_ij[2 * k], j = m.hund_ij[2 * k + 1];
-        e -= m.hund_v[k] * (static_cast<double>(num[i] * num[j]) + static_cast<double>(num[i + ns] * num[j + ns]));
-      }
-      double transfer = 0.0;
-      for (int w = 0; w < nwarp; ++w) transfer += rowq[w];
-      e += transfer;
-      const bool ok = fabs(ip) >= 1.0e-100 && isfinite(e);
       valid[sample] = ok ? 1 : 0;
-      eloc[sample] = ok ? e : 0.0;
-      double lp = 0.0;
-      for (int k = 0; k < m.nproj; ++k) lp += m.proj[k] * static_cast<double>(cnt[k]);
+      eloc[sample] = ok ? en : 0.0;
       lpsi[sample] = ok ? lp + log(fabs(ip)) : 0.0;
-      pf[m.nqp + 1] = ok ? 1.0 : 0.0;
     }
-    __syncthreads();
-    const bool ok = pf[m.nqp + 1] != 0.0;
     const double inv_ip = ip / (ip * ip);
     for (int k = tid; k < m.sr_size; k += nt) {
       double v;
       if (k == 0) v = 1.0;
       else if (k <= m.nproj) v = static_cast<double>(cnt[k - 1]);
-      else v = orow[k] * inv_ip;
+      else v = oacc[k - 1 - m.nproj] * inv_ip;
       orow[k] = ok ? v : 0.0;
     }
     __syncthreads();
   }
 }
 
-bool packed_measure_fits(const DevModel& m, int limit) {
-  return m.orb_off != nullptr && m.trans_inv != nullptr && m.n <= 256 &&
-         packed_layout(m).total <= static_cast<size_t>(limit);
+// Threads per sample of the tile measurement; 0 where it is not used: the planes do not fit, a
+// translation is not a permutation, or the model is small (up to four planes of side 64).
+// Small models keep the square planes and their digits: the SR-CG amplifies any change of
+// rounding in its operands (two measurements that agree to 1e-15 gave updates 1e-6 to 1e-3
+// apart), such models are the ones compared with other programs digit by digit, and there the
+// tiles saved a fifth of a measurement of a few per cent of the step. From eight planes of 64 on
+// they halve it (2D 8×8, 4096 samples: 11.1 → 4.9 ms), at n = 224 they quarter it (2048
+// samples: 24.3 → 6.2 ms).
+// Sides up to 64 take two warps per sample when the samples fill the SMs several times over;
+// fewer samples leave the SMs to the latency of one sample, which eight warps shorten.
+int tri_measure_threads(const DevModel& m, const MeasTables& mt, int nsamples, int limit) {
+  const bool small = m.n <= 64 && static_cast<long long>(m.nqp) * m.n * m.n < 8 * 64 * 64;
+  if (small || !mt.orb_ent || m.n > 224 || m.ns2 > 32767 || tri_layout(m, false).total + 512 > static_cast<size_t>(limit))
+    return 0;
+  const bool many = nsamples > 4 * current_device_attr(cudaDevAttrMultiProcessorCount);
+  return m.n <= 64 ? (many ? 64 : 256) : (m.n <= 128 ? 256 : 512);
 }
 
-template <int JPL>
-int launch_measure_packed(const DevModel& m, const int* s_idx, const int* s_cfg, const int* s_num, const int* s_cnt,
-                          int nsamples, double* gws, size_t gws_stride, int gws_blocks, double* ostore, double* eloc,
-                          double* lpsi, int* valid, unsigned* status, cudaStream_t stream) {
-  const size_t smem = packed_layout(m).total;
-  auto kernel = k_measure_packed<JPL>;
+template <int NT, int PG, int CPT>
+int launch_measure_tri(const DevModel& m, const MeasTables& mt, const int* s_idx, const int* s_cfg, const int* s_num,
+                       const int* s_cnt, int nsamples, double* gws, size_t gws_stride, int gws_blocks, double* ostore,
+                       double* eloc, double* lpsi, int* valid, unsigned* status, cudaStream_t stream, int limit) {
+  auto kernel = k_measure_tri<NT, PG, CPT>;
+  // the plane sums in shared memory where they take no more than a quarter of the rest
+  const size_t plain = tri_layout(m, false).total, with = tri_layout(m, true).total;
+  const int acc = with <= plain + plain / 4 && with + 512 <= static_cast<size_t>(limit) ? 1 : 0;
+  if (!acc && gws_stride < static_cast<size_t>(m.nterm)) return kErrArgument;
+  const size_t smem = acc ? with : plain;
   MVMCB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  const int grid = std::max(1, std::min({nsamples, gws_blocks, current_device_attr(cudaDevAttrMultiProcessorCount)}));
-  kernel<<<grid, kPackedThreads, smem, stream>>>(m, s_idx, s_cfg, s_num, s_cnt, nsamples, gws, gws_stride, ostore,
-                                                 eloc, lpsi, valid, status);
+  int per = 0;
+  MVMCB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, NT, smem));
+  int grid = std::min(nsamples, std::max(1, per) * current_device_attr(cudaDevAttrMultiProcessorCount));
+  if (!acc) grid = std::min(grid, gws_blocks);
+  kernel<<<std::max(1, grid), NT, smem, stream>>>(m, mt, s_idx, s_cfg, s_num, s_cnt, nsamples, acc, gws, gws_stride,
+                                                  ostore, eloc, lpsi, valid, status);
   MVMCB_CUDA(cudaGetLastError());
   return kOk;
 }
@@ -1024,10 +1020,7 @@ int launch_measure_jpl(const DevModel& m, const int* s_idx, const int* s_cfg, co
 
 
 // gval != nullptr selects the PhysCal form: Green rows [nsamples][m.gw] instead of O rows.
-// Planes that do not fit one SM's shared memory are swept as packed upper triangles in
-// shared memory (k_measure_packed) when those fit, else in place in each block's L2
-// workspace (MVMC_B200_MEASURE=l2 selects the latter).
-int launch_measure(const DevModel& m, const int* s_idx, const int* s_cfg, const int* s_num,
+int launch_measure(const DevModel& m, const MeasTables& mt, const int* s_idx, const int* s_cfg, const int* s_num,
                    const int* s_cnt, int nsamples, double* gws, int gws_blocks, double* ostore,
                    double* eloc, double* lpsi, int* valid, double* gval, unsigned* status, cudaStream_t stream) {
   int dev = 0, limit = 0;
@@ -1035,17 +1028,19 @@ int launch_measure(const DevModel& m, const int* s_idx, const int* s_cfg, const 
   cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   const int n = m.n;
   const char* mode = std::getenv("MVMC_B200_MEASURE");
-  // planes too large for shared memory whose upper triangle fits: the packed sweep
-  // (MVMC_B200_MEASURE=l2 keeps the in-place sweep of full planes in L2)
+  // O rows of larger models: the planes as tiles of the upper triangle (MVMC_B200_MEASURE=l2
+  // keeps square planes, in shared memory or in L2)
   const size_t gws_stride = static_cast<size_t>(2) * n * n;
-  if (!gval && meas_layout(m, true).total > static_cast<size_t>(limit) && packed_measure_fits(m, limit) &&
-      gws_stride >= static_cast<size_t>(2) * m.nterm && !(mode && std::strcmp(mode, "l2") == 0)) {
-    if (n <= 224)
-      return launch_measure_packed<7>(m, s_idx, s_cfg, s_num, s_cnt, nsamples, gws, gws_stride, gws_blocks, ostore,
-                                      eloc, lpsi, valid, status, stream);
-    return launch_measure_packed<8>(m, s_idx, s_cfg, s_num, s_cnt, nsamples, gws, gws_stride, gws_blocks, ostore,
-                                    eloc, lpsi, valid, status, stream);
-  }
+  const bool l2 = mode && std::strcmp(mode, "l2") == 0;
+  const int nt = gval || l2 ? 0 : tri_measure_threads(m, mt, nsamples, limit);
+#define MVMCB_MEASURE_TRI(NT, PG, C)                                                                                 \
+  launch_measure_tri<NT, PG, C>(m, mt, s_idx, s_cfg, s_num, s_cnt, nsamples, gws, gws_stride, gws_blocks, ostore, eloc, \
+                                lpsi, valid, status, stream, limit)
+  if (nt == 64) return MVMCB_MEASURE_TRI(64, 64, 1);
+  if (nt == 256 && n <= 64) return MVMCB_MEASURE_TRI(256, 64, 1);
+  if (nt == 256) return MVMCB_MEASURE_TRI(256, 128, 1);
+  if (nt == 512) return MVMCB_MEASURE_TRI(512, 256, 1);
+#undef MVMCB_MEASURE_TRI
 #define MVMCB_MEASURE(J) \
   launch_measure_jpl<J>(m, s_idx, s_cfg, s_num, s_cnt, nsamples, gws, gws_blocks, ostore, eloc, lpsi, valid, gval, \
                         status, stream, limit)

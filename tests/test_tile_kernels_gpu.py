@@ -1,0 +1,40 @@
+"""The tile-based measurement (planes as 8×8 tiles of the upper triangle) at the edges of its
+range: sides around multiples of 8, 32 and 64, one and several planes, few and many samples."""
+import numpy as np
+import pytest
+
+from mvmc_lib import lattice, mvmc
+
+pytestmark = pytest.mark.gpu
+
+
+def inputs(tmp_path, lx, ly, n_up, nmp=1, nsp=1, **kw):
+    shifts = [(0, 0), (1, 0), (0, 1), (1, 1)] if ly > 1 else [(0, 0), (1, 0), (2, 0), (3, 0)]
+    args = dict(n_up=n_up, nmp=nmp, nsp_gauss_leg=nsp, shifts=shifts, samples=2, warmup=2, interval=3)
+    args.update(kw)
+    return lattice().write_inputs(str(tmp_path), lx, ly, **args)[:2]
+
+
+@pytest.mark.parametrize("lx,ly,n_up,nmp,nsp,walkers", [
+    (8, 8, 32, 4, 2, 700),     # n = 64, eight planes: two warps per sample
+    (8, 8, 32, 4, 2, 40),      # the same, eight warps per sample
+    (9, 8, 33, 1, 2, 9),       # n = 66, 256 threads
+    (11, 12, 64, 1, 1, 9),     # n = 128
+    (11, 12, 65, 1, 1, 9),     # n = 130, 512 threads
+    (16, 14, 111, 1, 1, 9),    # n = 222
+])
+def test_tile_measurement_matches_the_square_planes(tmp_path, monkeypatch, lx, ly, n_up, nmp, nsp, walkers):
+    """O rows, energies and ln|Psi| of the same samples from tiles and from the in-place sweep
+    of square planes. Two sweeps of one plane differ by its condition number (below 1e5 here)
+    times the rounding of n/2 steps, 1e5 · 128 · 1e-16 ≈ 1e-9 relative."""
+    nl, init = inputs(tmp_path, lx, ly, n_up, nmp, nsp, interval=1, samples=1)
+    eng = mvmc().Engine(nl, initial_def=init, walkers=walkers, precision=64, seed=5)
+    eng.sample()
+    rows = {}
+    for mode in ("tiles", "l2"):
+        monkeypatch.setenv("MVMC_B200_MEASURE", mode)
+        e, ho, oo = eng.measure()
+        rows[mode] = (eng.o_store(), eng.local_energies(), eng.log_amplitudes(), e, ho, oo)
+    assert eng.status() == 0
+    for a, b in zip(rows["tiles"], rows["l2"]):
+        assert np.max(np.abs(a - b)) <= 1e-9 * max(1.0, np.max(np.abs(b)))

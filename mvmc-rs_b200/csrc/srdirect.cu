@@ -6,14 +6,15 @@
 // is one dgemm of the stored rows, c_order_gram_real :312), assemble_s_g (:484-511) and
 // cholesky_solve (sr.rs:535: LAPACK dpotrf('U') + dpotrs).
 //
-// K6 k_gram: OO = Σ_s O_s O_sᵀ / Wc over the stored rows, 64×64 output tiles of the lower
-// triangle per block (4×4 per thread), the sample axis staged through shared memory in
-// chunks of 16 rows; every entry is summed in sample order, then mirrored.
-// K7 k_cholesky: one cooperative launch, right-looking with 32-wide panels: block 0
-// factors the diagonal block in shared memory, all blocks solve the panel rows below it,
-// all blocks update the trailing lower triangle in 64×64 tiles (grid barrier between the
-// three). S = L Lᵀ with L = Uᵀ of dpotrf('U'). K8 k_cholesky_solve: one block, the
-// forward and backward substitutions blocked by 32.
+// K6 k_gram: OO = Σ_s O_s O_sᵀ / Wc over the stored rows on the FP64 tensor instruction
+// (mma.sync m8n8k4; tcgen05 has no FP64 kind): 64×64 output tiles of the lower triangle, one
+// per block of four warps, the sample axis through a three-stage cp.async ring, mirrored.
+// K7 k_cholesky: one cooperative launch, right-looking with 64-wide panels: all blocks solve
+// the panel rows below the diagonal block, then update the trailing lower triangle in 64×64
+// mma tiles; block 0 updates and factors the next diagonal block meanwhile, so a panel costs
+// two grid barriers. The right-hand side rides along as one more row, which makes it
+// y = L⁻¹b. S = L Lᵀ with L = Uᵀ of dpotrf('U'). K8 k_cholesky_back: Lᵀx = y, one grid barrier
+// per 64 unknowns.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -24,70 +25,106 @@
 #include "../../include/mvmc_b200.h"
 #include "../host/abi_common.h"
 #include "common.cuh"
+#include "skewtile.cuh"
 
 namespace cgr = cooperative_groups;
 
 namespace mvmcb {
 
 constexpr int kGramTile = 64;
-constexpr int kGramK = 16;
-constexpr int kCholB = 32;   // panel width
-constexpr int kCholT = 64;   // trailing-update tile (kCholThreads = 16 × 16 threads, 4 × 4 each)
+constexpr int kGramK = 16;       // samples per stage
+constexpr int kGramStages = 3;
+constexpr int kGramThreads = 128;
+constexpr int kGramLd = kGramTile + 4;  // ≡ 4 mod 16: a fragment's four rows in different banks
+constexpr int kCholB = 64;       // panel width and trailing-update tile
+constexpr int kCholLd = kCholB + 4;
 constexpr int kCholThreads = 256;
 
-// OO[i][j] (i ≥ j tiles) of the rows store[s][0..n) for s < ns, scaled by inv_w.
-__global__ void __launch_bounds__(256) k_gram(const double* __restrict__ store, int n, long long ns, double inv_w,
-                                              double* __restrict__ oo) {
-  __shared__ double As[kGramK][kGramTile + 1];
-  __shared__ double Bs[kGramK][kGramTile + 1];
-  const int ntile = (n + kGramTile - 1) / kGramTile;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  for (int t = blockIdx.x; t < ntile * (ntile + 1) / 2; t += gridDim.x) {
-    // triangular tile index → (ti, tj), ti ≥ tj
-    int ti = static_cast<int>((sqrt(8.0 * t + 1.0) - 1.0) / 2.0);
-    while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
-    while (ti * (ti + 1) / 2 > t) --ti;
-    const int tj = t - ti * (ti + 1) / 2;
-    const int i0 = ti * kGramTile, j0 = tj * kGramTile;
-    double acc[4][4];
+// Triangular tile index → (ti, tj), ti ≥ tj.
+__device__ __forceinline__ void tri_index(int t, int& ti, int& tj) {
+  ti = static_cast<int>((sqrt(8.0 * t + 1.0) - 1.0) / 2.0);
+  while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
+  while (ti * (ti + 1) / 2 > t) --ti;
+  tj = t - ti * (ti + 1) / 2;
+}
+
+// Eight bytes to shared memory without a register (rows of an odd number of doubles allow no
+// wider copy); zero where !on.
+__device__ __forceinline__ void cp_async8(double* dst, const double* src, bool on) {
+  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(on ? 8 : 0) : "memory");
+}
+
+// OO[i][j] (i ≥ j tiles) of the rows store[s][0..n) for s < ns, scaled by inv_w. A warp owns
+// 32×32 outputs as 4×4 accumulators: eight fragment loads for sixteen mma's, a quarter of the
+// shared-memory rate beside the full FP64 rate. Four blocks of 52 KB per SM: the 2278 tiles
+// of 4227 columns fill 3.85 waves of 592.
+__global__ void __launch_bounds__(kGramThreads, 4) k_gram(const double* __restrict__ store, int n, long long ns,
+                                                          double inv_w, double* __restrict__ oo) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  double* buf = reinterpret_cast<double*>(smem);  // [stage][A, B][kGramK][kGramLd]
+  constexpr int kHalf = kGramK * kGramLd, kStage = 2 * kHalf;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, k4 = lane & 3;
+  const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
+  int ti, tj;
+  tri_index(blockIdx.x, ti, tj);
+  const int i0 = ti * kGramTile, j0 = tj * kGramTile;
+  const long long chunks = (ns + kGramK - 1) / kGramK;
+  auto load = [&](long long c) {
+    double* dst = buf + static_cast<int>(c % kGramStages) * kStage;
+    const int col = tid & 63;
+    const bool ia = i0 + col < n, ja = j0 + col < n;
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
-    for (long long s0 = 0; s0 < ns; s0 += kGramK) {
-      for (int e = tid; e < kGramK * kGramTile; e += blockDim.x) {
-        const int r = e / kGramTile, c = e - r * kGramTile;
-        const long long s = s0 + r;
-        As[r][c] = (s < ns && i0 + c < n) ? store[s * n + i0 + c] : 0.0;
-        Bs[r][c] = (s < ns && j0 + c < n) ? store[s * n + j0 + c] : 0.0;
-      }
-      __syncthreads();
-#pragma unroll
-      for (int k = 0; k < kGramK; ++k) {
-        double av[4], bv[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) av[a] = As[k][ty + 16 * a];
-#pragma unroll
-        for (int b = 0; b < 4; ++b) bv[b] = Bs[k][tx + 16 * b];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b) acc[a][b] += av[a] * bv[b];
-      }
-      __syncthreads();
+    for (int e = 0; e < kGramK / 2; ++e) {
+      const int r = (tid >> 6) + 2 * e;
+      const long long s = c * kGramK + r;
+      const double* row = store + (s < ns ? s : 0) * n;
+      cp_async8(dst + r * kGramLd + col, row + (ia ? i0 + col : 0), ia && s < ns);
+      cp_async8(dst + kHalf + r * kGramLd + col, row + (ja ? j0 + col : 0), ja && s < ns);
     }
+  };
+  double acc[4][4][2];
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+  for (int a = 0; a < 4; ++a)
 #pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const int i = i0 + ty + 16 * a, j = j0 + tx + 16 * b;
+    for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+  for (int c = 0; c < kGramStages - 1; ++c) {
+    if (c < chunks) load(c);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  for (long long c = 0; c < chunks; ++c) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kGramStages - 2) : "memory");
+    __syncthreads();  // chunk c has arrived; chunk c − 1 has been read
+    if (c + kGramStages - 1 < chunks) load(c + kGramStages - 1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const double* A = buf + static_cast<int>(c % kGramStages) * kStage + k4 * kGramLd + wm + g;
+    const double* B = buf + static_cast<int>(c % kGramStages) * kStage + kHalf + k4 * kGramLd + wn + g;
+#pragma unroll
+    for (int k = 0; k < kGramK; k += 4) {
+      double av[4], bv[4];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) av[a] = A[k * kGramLd + 8 * a];
+#pragma unroll
+      for (int b = 0; b < 4; ++b) bv[b] = B[k * kGramLd + 8 * b];
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) dmma884(acc[a][b][0], acc[a][b][1], av[a], bv[b]);
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int i = i0 + wm + 8 * a + g, j = j0 + wn + 8 * b + 2 * k4 + h;
         if (i < n && j < n && i >= j) {
-          const double v = acc[a][b] * inv_w;
+          const double v = acc[a][b][h] * inv_w;
           oo[static_cast<size_t>(i) * n + j] = v;
           oo[static_cast<size_t>(j) * n + i] = v;
         }
       }
-  }
 }
 
 // S[si][sj] = OO[pi][pj] − OO[0][pi]·OO[0][pj] (pi = map[si] + 1), diagonal × (1 + sta_del).
@@ -120,184 +157,239 @@ __global__ void k_assemble_s_gram(const float* __restrict__ g, int ldg, const do
   }
 }
 
-// In-place lower Cholesky of the row-major n×n matrix a (the lower triangle is read and
-// written). info: 0, or the 1-based row of the first non-positive / non-finite pivot.
-__global__ void __launch_bounds__(kCholThreads) k_cholesky(double* __restrict__ a, int n, int* info) {
-  cgr::grid_group grid = cgr::this_grid();
-  __shared__ double D[kCholB][kCholB + 1];
-  __shared__ double Ti[kCholT][kCholB + 1];
-  __shared__ double Tj[kCholT][kCholB + 1];
-  __shared__ int s_fail;
+// Factor of the kb×kb diagonal block in D (lower, in place) by the whole block. fail: 1-based
+// column of the first non-positive or non-finite pivot, 0 none (such a pivot counts as 1).
+__device__ int factor_diagonal(double (*D)[kCholLd], int kb) {
   const int tid = threadIdx.x, nt = blockDim.x;
-  for (int k0 = 0; k0 < n; k0 += kCholB) {
-    const int kb = min(kCholB, n - k0);
-    // (1) diagonal block
-    if (blockIdx.x == 0) {
-      for (int e = tid; e < kb * kb; e += nt) {
-        const int r = e / kb, c = e - r * kb;
-        D[r][c] = c <= r ? a[static_cast<size_t>(k0 + r) * n + k0 + c] : 0.0;
-      }
-      if (tid == 0) s_fail = 0;
-      __syncthreads();
-      for (int j = 0; j < kb; ++j) {
-        if (tid == 0) {
-          double d = D[j][j];
-          for (int k = 0; k < j; ++k) d -= D[j][k] * D[j][k];
-          if (!(d > 0.0) || !isfinite(d)) {
-            if (!s_fail) s_fail = k0 + j + 1;
-            d = 1.0;
-          }
-          D[j][j] = sqrt(d);
-        }
-        __syncthreads();
-        for (int i = j + 1 + tid; i < kb; i += nt) {
-          double t = D[i][j];
-          for (int k = 0; k < j; ++k) t -= D[i][k] * D[j][k];
-          D[i][j] = t / D[j][j];
-        }
-        __syncthreads();
-      }
-      for (int e = tid; e < kb * kb; e += nt) {
-        const int r = e / kb, c = e - r * kb;
-        if (c <= r) a[static_cast<size_t>(k0 + r) * n + k0 + c] = D[r][c];
-      }
-      if (tid == 0 && s_fail && *info == 0) *info = s_fail;
+  int fail = 0;
+  for (int j = 0; j < kb; ++j) {
+    double d = D[j][j];
+    if (!(d > 0.0) || !isfinite(d)) {  // the same value in every thread
+      if (!fail) fail = j + 1;
+      d = 1.0;
     }
-    grid.sync();
-    if (*info != 0) return;  // every block reads the same flag after the barrier
-    const int rest = n - k0 - kb;
-    if (rest <= 0) break;
-    // (2) panel rows below: L[i][k0..k0+kb) = A[i][k0..) · D⁻ᵀ
-    for (int e = tid; e < kb * kb; e += nt) {
-      const int r = e / kb, c = e - r * kb;
-      D[r][c] = c <= r ? a[static_cast<size_t>(k0 + r) * n + k0 + c] : 0.0;
+    d = sqrt(d);
+    const double rd = 1.0 / d;
+    __syncthreads();  // D[j][j] read
+    for (int i = j + tid; i < kb; i += nt) D[i][j] = i == j ? d : D[i][j] * rd;
+    __syncthreads();
+    // sixteen threads per row of the trailing block
+    for (int i = j + 1 + tid / 16; i < kb; i += nt / 16) {
+      const double lij = D[i][j];
+      for (int c = j + 1 + tid % 16; c <= i; c += 16) D[i][c] -= lij * D[c][j];
     }
     __syncthreads();
-    for (int r = blockIdx.x * nt + tid; r < rest; r += gridDim.x * nt) {
-      double* row = a + static_cast<size_t>(k0 + kb + r) * n + k0;
-      double x[kCholB];
-#pragma unroll
-      for (int j = 0; j < kCholB; ++j) {
-        if (j < kb) {
-          double t = row[j];
-          for (int k = 0; k < j; ++k) t -= x[k] * D[j][k];
-          x[j] = t / D[j][j];
-        }
+  }
+  return fail;
+}
+
+// In-place lower Cholesky of the row-major n×n matrix a (the lower triangle is read and
+// written) with b as row n: b becomes L⁻¹b. info: 0, or the 1-based row of the first
+// non-positive / non-finite pivot.
+__global__ void __launch_bounds__(kCholThreads, 2) k_cholesky(double* __restrict__ a, int n, double* __restrict__ b,
+                                                              int* info) {
+  cgr::grid_group grid = cgr::this_grid();
+  extern __shared__ __align__(16) unsigned char smem[];
+  double(*Li)[kCholLd] = reinterpret_cast<double(*)[kCholLd]>(smem);
+  double(*Lj)[kCholLd] = Li + kCholB;
+  __shared__ double rdiag[kCholB];
+  const int tid = threadIdx.x, nt = kCholThreads, lane = tid & 31, warp = tid >> 5, g = lane >> 2, k4 = lane & 3;
+  auto row_of = [&](int r) { return r < n ? a + static_cast<size_t>(r) * n : b; };
+  // block 0: factor the diagonal block at k (in Li, or read from a) and store it
+  auto diagonal = [&](int k, bool loaded) {
+    const int kb = min(kCholB, n - k);
+    if (!loaded)
+      for (int e = tid; e < kb * kb; e += nt) {
+        const int r = e / kb, c = e - r * kb;
+        Li[r][c] = c <= r ? a[static_cast<size_t>(k + r) * n + k + c] : 0.0;
       }
-#pragma unroll
-      for (int j = 0; j < kCholB; ++j)
-        if (j < kb) row[j] = x[j];
+    __syncthreads();
+    const int fail = factor_diagonal(Li, kb);
+    for (int e = tid; e < kb * kb; e += nt) {
+      const int r = e / kb, c = e - r * kb;
+      if (c <= r) a[static_cast<size_t>(k + r) * n + k + c] = Li[r][c];
     }
+    if (tid == 0 && fail && *info == 0) *info = k + fail;
+    __syncthreads();
+  };
+  if (blockIdx.x == 0) diagonal(0, false);
+  grid.sync();
+  for (int k0 = 0; k0 < n; k0 += kCholB) {
+    if (*reinterpret_cast<volatile int*>(info) != 0) return;  // every block reads the same flag after the barrier
+    const int kb = min(kCholB, n - k0), top = k0 + kb;
+    const int rest = n + 1 - top;  // rows below, the right-hand side among them
+    // (1) panel rows: L[i][k0..) = A[i][k0..)·D⁻ᵀ, 32 rows per block, eight lanes per row, eight
+    // columns at a time: the finished columns' products, then the 8×8 triangle by shuffles
+    if (blockIdx.x * 32 < rest) {
+      for (int e = tid; e < kCholB * kCholB; e += nt) {
+        const int r = e / kCholB, c = e % kCholB;
+        Li[r][c] = r < kb && c <= r ? a[static_cast<size_t>(k0 + r) * n + k0 + c] : (r == c ? 1.0 : 0.0);
+      }
+      __syncthreads();
+      if (tid < kCholB) rdiag[tid] = 1.0 / Li[tid][tid];
+      for (int r0 = blockIdx.x * 32; r0 < rest; r0 += gridDim.x * 32) {
+        __syncthreads();
+        for (int e = tid; e < 32 * kCholB; e += nt) {
+          const int r = e / kCholB, c = e % kCholB;
+          Lj[r][c] = r0 + r < rest && c < kb ? row_of(top + r0 + r)[k0 + c] : 0.0;
+        }
+        __syncthreads();
+        double* x = Lj[warp * 4 + (lane >> 3)];
+        const int c8 = lane & 7;
+        for (int jb = 0; jb < kCholB; jb += 8) {
+          const int j = jb + c8;
+          double t0 = x[j], t1 = 0.0;
+          for (int k = 0; k < jb; k += 2) {
+            t0 -= x[k] * Li[j][k];
+            t1 -= x[k + 1] * Li[j][k + 1];
+          }
+          double t = t0 + t1;
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const double xc = __shfl_sync(0xffffffffu, t * rdiag[jb + c8], c, 8);
+            if (c8 == c) t = xc;
+            if (c8 > c) t -= xc * Li[j][jb + c];
+          }
+          __syncwarp();
+          x[j] = t;
+          __syncwarp();
+        }
+        __syncthreads();
+        for (int e = tid; e < 32 * kCholB; e += nt) {
+          const int r = e / kCholB, c = e % kCholB;
+          if (r0 + r < rest && c < kb) row_of(top + r0 + r)[k0 + c] = Lj[r][c];
+        }
+      }
+    }
+    if (top >= n) break;  // only the right-hand side was left
     grid.sync();
-    // (3) trailing update of the lower triangle in 64×64 tiles (4×4 outputs per thread,
-    // the tile's two 64×32 panel slices staged in shared memory)
-    const int m = (rest + kCholT - 1) / kCholT;
-    const int ntiles = m * (m + 1) / 2;
-    const int tr = tid / 16, tc = tid % 16;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-      int ti = static_cast<int>((sqrt(8.0 * t + 1.0) - 1.0) / 2.0);
-      while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
-      while (ti * (ti + 1) / 2 > t) --ti;
-      const int tj = t - ti * (ti + 1) / 2;
-      const int i0 = k0 + kb + ti * kCholT, j0 = k0 + kb + tj * kCholT;
-      for (int e = tid; e < kCholT * kCholB; e += nt) {
-        const int r = e / kCholB, c = e - r * kCholB;
-        Ti[r][c] = (i0 + r < n && c < kb) ? a[static_cast<size_t>(i0 + r) * n + k0 + c] : 0.0;
-        Tj[r][c] = (j0 + r < n && c < kb) ? a[static_cast<size_t>(j0 + r) * n + k0 + c] : 0.0;
-      }
+    // (2) trailing update of the lower triangle and of the right-hand side in 64×64 tiles
+    const int mt = (rest + kCholB - 1) / kCholB;
+    const int ntiles = mt * (mt + 1) / 2;
+    const int wm = (warp >> 1) * 16, wn = (warp & 1) * 32;
+    const int step = max(1, static_cast<int>(gridDim.x) - 1);
+    for (int t = gridDim.x == 1 ? 0 : (blockIdx.x == 0 ? 0 : static_cast<int>(blockIdx.x)); t < ntiles;
+         t += blockIdx.x == 0 && gridDim.x > 1 ? ntiles : step) {
+      int ti, tj;
+      tri_index(t, ti, tj);
+      const int i0 = top + ti * kCholB, j0 = top + tj * kCholB;
+      if (j0 >= n) continue;
       __syncthreads();
-      double acc[4][4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) acc[u][v] = 0.0;
-#pragma unroll 8
-      for (int k = 0; k < kCholB; ++k) {
-        double li[4], lj[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          li[u] = Ti[tr + 16 * u][k];
-          lj[u] = Tj[tc + 16 * u][k];
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int v = 0; v < 4; ++v) acc[u][v] += li[u] * lj[v];
+      for (int e = tid; e < kCholB * kCholB; e += nt) {
+        const int r = e / kCholB, c = e % kCholB;
+        const bool on = c < kb;
+        Li[r][c] = on && i0 + r <= n ? __ldcg(row_of(i0 + r) + k0 + c) : 0.0;
+        Lj[r][c] = on && j0 + r < n ? __ldcg(a + static_cast<size_t>(j0 + r) * n + k0 + c) : 0.0;
       }
+      double acc[2][4][2];
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
+      for (int u = 0; u < 2; ++u)
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          const int i = i0 + tr + 16 * u, j = j0 + tc + 16 * v;
-          if (i < n && j < n && j <= i) a[static_cast<size_t>(i) * n + j] -= acc[u][v];
-        }
+        for (int v = 0; v < 4; ++v)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int i = i0 + wm + 8 * u + g, j = j0 + wn + 8 * v + 2 * k4 + h;
+            acc[u][v][h] = i <= n && j < n && j <= i ? __ldcg(row_of(i) + j) : 0.0;
+          }
       __syncthreads();
+#pragma unroll 4
+      for (int k = 0; k < kCholB; k += 4) {
+        double av[2], bv[4];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) av[u] = -Li[wm + 8 * u + g][k + k4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) bv[v] = Lj[wn + 8 * v + g][k + k4];
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int v = 0; v < 4; ++v) dmma884(acc[u][v][0], acc[u][v][1], av[u], bv[v]);
+      }
+      const bool next_diagonal = t == 0;
+      if (next_diagonal) __syncthreads();  // Li is rewritten below
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int r = wm + 8 * u + g, c = wn + 8 * v + 2 * k4 + h, i = i0 + r, j = j0 + c;
+            if (next_diagonal && i < n && j < n) Li[r][c] = j <= i ? acc[u][v][h] : 0.0;
+            else if (i <= n && j < n && j <= i) row_of(i)[j] = acc[u][v][h];
+          }
+      if (next_diagonal) diagonal(top, true);
     }
     grid.sync();
   }
 }
 
-// x = (L Lᵀ)⁻¹ b in place, L the lower factor of k_cholesky; one block.
-__global__ void __launch_bounds__(kCholThreads) k_cholesky_solve(const double* __restrict__ l, int n,
-                                                                 double* __restrict__ b) {
-  __shared__ double part[kCholThreads / kCholB][kCholB];
-  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31;
-  // forward: L y = b
-  for (int k0 = 0; k0 < n; k0 += kCholB) {
+// x = L⁻ᵀ y in place (b), L the lower factor: from the last 64 unknowns up, every block solves
+// the 64×64 triangle itself and takes 32 of the columns still to be updated per pass.
+__global__ void __launch_bounds__(kCholThreads) k_cholesky_back(const double* __restrict__ l, int n,
+                                                                double* __restrict__ b, const int* info) {
+  cgr::grid_group grid = cgr::this_grid();
+  __shared__ double D[kCholB][kCholB + 1];
+  __shared__ double x[kCholB];
+  __shared__ double part[kCholThreads / 32][32];
+  if (*info != 0) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int kWarps = kCholThreads / 32;
+  for (int k0 = (n - 1) / kCholB * kCholB; k0 >= 0; k0 -= kCholB) {
     const int kb = min(kCholB, n - k0);
-    if (tid < 32) {
-      double y = lane < kb ? b[k0 + lane] : 0.0;
-      for (int j = 0; j < kb; ++j) {
-        if (lane == j) y = y / l[static_cast<size_t>(k0 + j) * n + k0 + j];
-        const double yj = __shfl_sync(0xffffffffu, y, j);
-        if (lane > j && lane < kb) y -= l[static_cast<size_t>(k0 + lane) * n + k0 + j] * yj;
-      }
-      if (lane < kb) b[k0 + lane] = y;
+    for (int e = tid; e < kCholB * kCholB; e += kCholThreads) {
+      const int r = e / kCholB, c = e % kCholB;
+      D[r][c] = r < kb && c <= r ? l[static_cast<size_t>(k0 + r) * n + k0 + c] : (r == c ? 1.0 : 0.0);
     }
     __syncthreads();
-    for (int i = k0 + kb + tid; i < n; i += nt) {
+    if (warp == 0) {
+      double y0 = lane < kb ? __ldcg(b + k0 + lane) : 0.0, y1 = lane + 32 < kb ? __ldcg(b + k0 + lane + 32) : 0.0;
+      const double r0 = 1.0 / D[lane][lane], r1 = 1.0 / D[lane + 32][lane + 32];
+#pragma unroll 8
+      for (int j = kCholB - 1; j >= 32; --j) {
+        const double xj = __shfl_sync(0xffffffffu, y1 * r1, j - 32);
+        if (lane + 32 == j) y1 = xj;
+        if (lane + 32 < j) y1 -= D[j][lane + 32] * xj;
+        y0 -= D[j][lane] * xj;
+      }
+#pragma unroll 8
+      for (int j = 31; j >= 0; --j) {
+        const double xj = __shfl_sync(0xffffffffu, y0 * r0, j);
+        if (lane == j) y0 = xj;
+        if (lane < j) y0 -= D[j][lane] * xj;
+      }
+      x[lane] = y0;
+      x[lane + 32] = y1;
+    }
+    __syncthreads();
+    for (int c0 = blockIdx.x * 32; c0 < k0; c0 += gridDim.x * 32) {
+      const int c = c0 + lane;
       double t = 0.0;
-      const double* row = l + static_cast<size_t>(i) * n + k0;
-      for (int k = 0; k < kb; ++k) t += row[k] * b[k0 + k];
-      b[i] -= t;
-    }
-    __syncthreads();
-  }
-  // backward: Lᵀ x = y, blocks from the bottom
-  const int nb = (n + kCholB - 1) / kCholB;
-  for (int bi = nb - 1; bi >= 0; --bi) {
-    const int k0 = bi * kCholB, kb = min(kCholB, n - k0), below = k0 + kb;
-    // y_J −= Σ_{i ≥ below} L[i][J] x_i: column j = tid % 32, row groups by tid / 32
-    {
-      const int j = tid % kCholB, grp = tid / kCholB, ngrp = nt / kCholB;
-      double t = 0.0;
-      if (j < kb)
-        for (int i = below + grp; i < n; i += ngrp) t += l[static_cast<size_t>(i) * n + k0 + j] * b[i];
-      part[grp][j] = t;
-    }
-    __syncthreads();
-    if (tid < 32) {
-      double x = 0.0;
-      if (lane < kb) {
-        double t = 0.0;
-        for (int g = 0; g < nt / kCholB; ++g) t += part[g][lane];
-        x = b[k0 + lane] - t;
+      if (c < k0) {
+#pragma unroll
+        for (int r = 0; r < kCholB / kWarps; ++r) {
+          const int rr = warp * (kCholB / kWarps) + r;
+          if (rr < kb) t += l[static_cast<size_t>(k0 + rr) * n + c] * x[rr];
+        }
       }
-      for (int j = kb - 1; j >= 0; --j) {
-        if (lane == j) x = x / l[static_cast<size_t>(k0 + j) * n + k0 + j];
-        const double xj = __shfl_sync(0xffffffffu, x, j);
-        if (lane < j) x -= l[static_cast<size_t>(k0 + j) * n + k0 + lane] * xj;
+      part[warp][lane] = t;
+      __syncthreads();
+      if (warp == 0 && c < k0) {
+        double s = 0.0;
+        for (int u = 0; u < kWarps; ++u) s += part[u][lane];
+        b[c] = __ldcg(b + c) - s;
       }
-      if (lane < kb) b[k0 + lane] = x;
+      __syncthreads();
     }
+    grid.sync();  // the blocks have read their y before block 0 puts x there
+    if (blockIdx.x == 0 && tid < kb) b[k0 + tid] = x[tid];
     __syncthreads();
   }
 }
 
 int launch_gram(const double* store, int n, long long ns, double inv_w, double* oo, cudaStream_t stream) {
   const int ntile = (n + kGramTile - 1) / kGramTile;
-  const int tiles = ntile * (ntile + 1) / 2;
-  k_gram<<<std::max(1, std::min(tiles, 148 * 8)), 256, 0, stream>>>(store, n, ns, inv_w, oo);
+  const size_t smem = sizeof(double) * kGramStages * 2 * kGramK * kGramLd;
+  MVMCB_CUDA(cudaFuncSetAttribute(k_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  k_gram<<<ntile * (ntile + 1) / 2, kGramThreads, smem, stream>>>(store, n, ns, inv_w, oo);
   MVMCB_CUDA(cudaGetLastError());
   return kOk;
 }
@@ -322,17 +414,20 @@ int launch_assemble_s_gram(const float* g, int ldg, const double* cs, const doub
 
 // Factor a (n×n, device) and solve for b (device) in place; *info_dev set on failure.
 int launch_cholesky_solve(double* a, int n, double* b, int* info_dev, cudaStream_t stream) {
-  int dev = 0, sms = 0, per = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  MVMCB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cholesky, kCholThreads, 0));
-  const int m = (n + kCholB - 1) / kCholB;
-  const int blocks = std::max(1, std::min(sms * std::max(1, std::min(per, 2)), m * (m + 1) / 2));
+  const size_t smem = sizeof(double) * 2 * kCholB * kCholLd;
+  MVMCB_CUDA(cudaFuncSetAttribute(k_cholesky, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  int per = 0;
+  MVMCB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cholesky, kCholThreads, smem));
+  const int sms = current_device_attr(cudaDevAttrMultiProcessorCount);
+  const int m = (n + kCholB) / kCholB;  // tile rows, the right-hand side's row among them
+  // block 0 takes the next diagonal block, the others the rest of a step's tiles
+  const int blocks = std::max(1, std::min(sms * std::max(1, std::min(per, 2)), m * (m + 1) / 2 + 1));
   MVMCB_CUDA(cudaMemsetAsync(info_dev, 0, sizeof(int), stream));
-  void* args[] = {&a, &n, &info_dev};
-  MVMCB_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k_cholesky), blocks, kCholThreads, args, 0, stream));
-  k_cholesky_solve<<<1, kCholThreads, 0, stream>>>(a, n, b);
-  MVMCB_CUDA(cudaGetLastError());
+  void* args[] = {&a, &n, &b, &info_dev};
+  MVMCB_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k_cholesky), blocks, kCholThreads, args, smem, stream));
+  void* back[] = {&a, &n, &b, &info_dev};
+  MVMCB_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k_cholesky_back), std::max(1, std::min(sms, (n + 31) / 32)),
+                                         kCholThreads, back, 0, stream));
   return kOk;
 }
 

@@ -109,3 +109,39 @@ def test_direct_sr_through_tensor_core_gram(tmp_path, sr_precision, bound):
     assert np.linalg.norm(d64) > 0
     err = np.linalg.norm(d - d64) / np.linalg.norm(d64)
     assert err <= bound, err
+
+
+@pytest.mark.parametrize("n,samples", [(1, 1), (63, 15), (64, 16), (65, 17), (129, 49), (130, 0)])
+def test_gram_at_tile_and_stage_edges(n, samples):
+    """64-column tiles, stages of 16 samples (fewer, one and several stages of the ring of
+    three, a remainder), an empty store; each entry within the rounding of its own sum."""
+    rng = np.random.default_rng(n)
+    store = rng.normal(size=(samples, n))
+    got = mvmc().gram(store)
+    bound = 4 * (samples + 1) * np.finfo(float).eps * (np.abs(store).T @ np.abs(store))
+    assert np.all(np.abs(got - store.T @ store) <= bound)
+    assert np.array_equal(got, got.T)
+
+
+@pytest.mark.parametrize("n", [31, 63, 64, 65, 127, 128, 129, 1100])
+def test_cholesky_solve_at_panel_edges(n):
+    """64-wide panels: a partial, one, and several panels, the right-hand side's row alone in
+    its tile (n a multiple of 64) or beside others. The residual is bounded by the
+    factorisation's backward error, n · eps · |S| · |x|, with a factor 8."""
+    rng = np.random.default_rng(n)
+    m = rng.normal(size=(n, n))
+    a = m @ m.T / n + 0.1 * np.eye(n)
+    b = rng.normal(size=n)
+    rc, x = mvmc().cholesky_solve(a, b)
+    assert rc == 0
+    bound = 8 * n * np.finfo(float).eps * np.linalg.norm(a, 2) * np.linalg.norm(x)
+    assert np.linalg.norm(a @ x - b) <= bound
+
+
+@pytest.mark.parametrize("n,at", [(64, 63), (65, 64), (200, 0), (200, 130)])
+def test_cholesky_solve_reports_a_bad_pivot_in_any_panel(n, at):
+    for bad in (-2.0, 0.0, np.nan, np.inf):
+        a = np.eye(n)
+        a[at, at] = bad
+        rc, _ = mvmc().cholesky_solve(a, np.ones(n))
+        assert rc == 1, bad

@@ -21,6 +21,8 @@ namespace mvmcb {
 
 int launch_sample(const DevModel& m, const DevWalkers& w, int precision, cudaStream_t stream);
 bool sample_planes_in_smem(const DevModel& m, int precision, int limit);
+bool sample_tri_applies(const DevModel& m, int precision, int limit);
+int launch_sample_tri(const DevModel& m, const DevWalkers& w, int precision, int limit, cudaStream_t stream);
 int launch_measure(const DevModel& m, const MeasTables& mt, const int* s_idx, const int* s_cfg, const int* s_num,
                    const int* s_cnt, int nsamples, double* gws, int gws_blocks, double* ostore,
                    double* eloc, double* lpsi, int* valid, double* gval, unsigned* status, cudaStream_t stream);
@@ -116,6 +118,8 @@ struct mvmc_b200_ctx {
   DevModel dm{};
   DevWalkers dw{};
   MeasTables mt{};
+  bool tri_sample = false;  // the FP64 sampler on tiles (sampler_tri.cu)
+  int smem_limit = 0;
   std::vector<void*> allocs;
   double* d_f = nullptr;
   double* d_proj = nullptr;
@@ -547,7 +551,9 @@ void build_context(mvmc_b200_ctx* c, const char* namelist, const char* initial_d
   cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const size_t nn = static_cast<size_t>(n) * n;
-  const bool smem = sample_planes_in_smem(dm, opt.precision, limit);
+  c->tri_sample = sample_tri_applies(dm, opt.precision, limit);
+  c->smem_limit = limit;
+  const bool smem = c->tri_sample || sample_planes_in_smem(dm, opt.precision, limit);
   dw.inv = nullptr;
   dw.ws64 = nullptr;
   if (!smem) {
@@ -592,6 +598,11 @@ int guarded(F&& f) {
     if (what.find("cuda") != std::string::npos || what.find("CUDA") != std::string::npos) return MVMC_B200_ECUDA;
     return MVMC_B200_EMODEL;
   }
+}
+
+int run_sampler(mvmc_b200_ctx* c) {
+  return c->tri_sample ? launch_sample_tri(c->dm, c->dw, c->opt.precision, c->smem_limit, c->stream)
+                       : launch_sample(c->dm, c->dw, c->opt.precision, c->stream);
 }
 
 int do_measure(mvmc_b200_ctx* c) {
@@ -1064,7 +1075,7 @@ extern "C" int mvmc_b200_set_parameters(mvmc_b200_ctx* c, const double* params, 
 extern "C" int mvmc_b200_sample(mvmc_b200_ctx* c) {
   if (!c) return MVMC_B200_EARG;
   return guarded([&]() {
-    int rc = launch_sample(c->dm, c->dw, c->opt.precision, c->stream);
+    int rc = run_sampler(c);
     if (rc != kOk) return rc;
     check(cudaStreamSynchronize(c->stream), "sample");
     c->sampled = true;
@@ -1220,7 +1231,7 @@ extern "C" int mvmc_b200_run_opt(const char* namelist, const char* initial_def, 
     std::vector<mvmc::OptPoint> window;
     bool first_info = true;
     for (int step = 0; step < m.nsr_opt_itr_step; ++step) {
-      int r = launch_sample(c->dm, c->dw, c->opt.precision, c->stream);
+      int r = run_sampler(c);
       if (r != kOk) return r;
       c->sampled = true;
       r = do_measure(c);
@@ -1301,7 +1312,7 @@ extern "C" int mvmc_b200_run_physcal(const char* namelist, const char* zqp_opt, 
   rc = guarded([&]() {
     const mvmc::Model& m = c->m;
     for (int b = 0; b < std::max(0, m.data_qty_smp); ++b) {
-      int r = launch_sample(c->dm, c->dw, c->opt.precision, c->stream);
+      int r = run_sampler(c);
       if (r != kOk) return r;
       c->sampled = true;
       std::vector<double> g;

@@ -1,4 +1,5 @@
-// K2: resident Metropolis sampler (one CTA per walker).
+// K2: resident Metropolis sampler (one CTA per walker) on square planes: the FP32 path, and the
+// FP64 walkers whose planes do not fit one SM as tiles (those that do run in sampler_tri.cu).
 //
 // Reproduces vmc_make_sample_real_engine (crates/mvmc-core/src/sampling/driver.rs:175-438)
 // and HostEngine::run_block (sampling/engine.rs:188-476) of AtelierArith/mvmc-rs for the
@@ -23,6 +24,7 @@
 #include "common.cuh"
 #include "engine.cuh"
 #include "pfinv.cuh"
+#include "sampler_common.cuh"
 #include "sfmt.cuh"
 
 namespace mvmcb {
@@ -105,26 +107,6 @@ __device__ __forceinline__ float slater_at<float>(const DevModel& m, int q, int 
   return __ldg(m.slater32 + (static_cast<size_t>(q) * m.ns2 + r1) * m.ns2 + r2);
 }
 
-// ---- projection counters --------------------------------------------------------------
-__device__ void make_proj_cnt_serial(const DevModel& m, const int* num, int* cnt) {
-  for (int k = 0; k < m.nproj; ++k) cnt[k] = 0;
-  for (int ri = 0; ri < m.ns; ++ri) {
-    const int g = m.gutz_idx[ri];
-    if (m.n_gutz > 0 && g >= 0 && g < m.nproj) cnt[g] += num[ri] * num[ri + m.ns];
-  }
-  if (m.n_jast > 0)
-    for (int ri = 0; ri < m.ns; ++ri) {
-      const int xi = num[ri] + num[ri + m.ns] - 1;
-      if (xi == 0) continue;
-      for (int rj = ri + 1; rj < m.ns; ++rj) {
-        const int j = __ldg(m.jast_idx + ri * m.ns + rj);
-        if (j < 0) continue;
-        const int xj = num[rj] + num[rj + m.ns] - 1;
-        if (m.n_gutz + j < m.nproj) cnt[m.n_gutz + j] += xi * xj;
-      }
-    }
-}
-
 // Δ ln P of a hop from `source` to `dest` by one warp, `num` holding the configuration
 // after the move: the direct-table form of Σ_k α_k (c'_k − c_k) (gutz_site[r] = α of r's
 // Gutzwiller class, jast_pair[a·ns + b] = α of the Jastrow class of (a, b); the form of the
@@ -156,33 +138,6 @@ __device__ __forceinline__ double log_proj_ratio_hop_warp(const DevModel& m, con
     z += __ldg(m.jast_pair + static_cast<size_t>(source) * ns + dest) * static_cast<double>(xs - xd + 1);
   }
   return z;
-}
-
-// Projection counters from the configuration by the whole CTA (make_proj_cnt,
-// projection.rs:179): integer sums, so the order of the atomics does not matter.
-__device__ void make_proj_cnt_cta(const DevModel& m, const int* jtab, const int* num, int* cnt) {
-  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarp = nt >> 5;
-  const int ns = m.ns;
-  for (int k = tid; k < m.nproj; k += nt) cnt[k] = 0;
-  __syncthreads();
-  if (m.n_gutz > 0)
-    for (int r = tid; r < ns; r += nt) {
-      const int g = m.gutz_idx[r];
-      const int v = num[r] * num[r + ns];
-      if (v && g >= 0 && g < m.nproj) atomicAdd(cnt + g, v);
-    }
-  if (m.n_jast > 0)
-    for (int ri = warp; ri < ns; ri += nwarp) {
-      const int xi = num[ri] + num[ri + ns] - 1;
-      if (xi == 0) continue;
-      for (int rj = ri + 1 + lane; rj < ns; rj += 32) {
-        const int j = jtab[ri * ns + rj];
-        if (j < 0) continue;
-        const int xj = num[rj] + num[rj + ns] - 1;
-        if (xj != 0 && m.n_gutz + j < m.nproj) atomicAdd(cnt + m.n_gutz + j, xi * xj);
-      }
-    }
-  __syncthreads();
 }
 
 // ---- CalculateMAll on every plane (CTA-wide); returns 0 ok, else the first failure -------
@@ -235,12 +190,6 @@ __device__ int calc_m_all_dev(const DevModel& m, const WalkerSmem<T>& s, unsigne
   }
   __syncthreads();
   return info;
-}
-
-__device__ __forceinline__ double log_ip_of(const DevModel& m, const double* pf, const double* qpw) {
-  double ip = 0.0;
-  for (int q = 0; q < m.nqp; ++q) ip += qpw[q] * pf[q];
-  return log(fabs(ip));
 }
 
 // ---- Pfaffian ratio of a hop: pf_new[q] = -pf[q]·Σ_j InvM[q][msa][j]·S_q[rsa][rs_j] --------
@@ -674,47 +623,6 @@ __device__ void update_exchange_dev(const DevModel& m, const WalkerSmem<T>& s, i
   __syncthreads();
 }
 
-// ---- serial helpers for thread 0 ------------------------------------------------------------
-__device__ __forceinline__ void move_electron(const DevModel& m, int* idx, int* cfg, int* num, int mi,
-                                              int ri, int rj, int sp) {
-  const int msa = mi + sp * m.ne, ro = ri + sp * m.ns, rn = rj + sp * m.ns;
-  idx[msa] = rj;
-  cfg[ro] = -1;
-  cfg[rn] = mi;
-  num[ro] = 0;
-  num[rn] = 1;
-}
-__device__ __forceinline__ void revert_electron(const DevModel& m, int* idx, int* cfg, int* num, int mi,
-                                                int ri, int rj, int sp) {
-  const int msa = mi + sp * m.ne, ro = ri + sp * m.ns, rn = rj + sp * m.ns;
-  idx[msa] = ri;
-  cfg[ro] = mi;
-  cfg[rn] = -1;
-  num[ro] = 1;
-  num[rn] = 0;
-}
-
-__device__ void make_initial_sample_dev(const DevModel& m, SfmtRef& rng, int* idx, int* cfg, int* num,
-                                        int* cnt) {
-  for (int k = 0; k < m.n; ++k) idx[k] = -1;
-  for (int k = 0; k < m.ns2; ++k) cfg[k] = -1;
-  for (int si = 0; si < 2; ++si)
-    for (int mi = 0; mi < m.ne; ++mi) {
-      int guard = 0;
-      while (true) {
-        const int ri = static_cast<int>(rng.mod(m.ns));
-        if (cfg[ri + si * m.ns] == -1) {
-          cfg[ri + si * m.ns] = mi;
-          idx[mi + si * m.ne] = ri;
-          break;
-        }
-        if (++guard > (1 << 24)) break;  // unreachable for ne <= nsite
-      }
-    }
-  for (int r = 0; r < m.ns2; ++r) num[r] = cfg[r] < 0 ? 0 : 1;
-  make_proj_cnt_serial(m, num, cnt);
-}
-
 // Walkers per SM the register budget is sized for: one when the planes are in shared
 // memory; with planes in L2, enough CTAs for 16 warps per SM (a tighter budget spills).
 template <int NT, bool kSmemPlanes>
@@ -1096,7 +1004,7 @@ bool sample_planes_in_smem(const DevModel& m, int precision, int limit) {
   if (precision == 32 && fp32_prefers_l2(m)) return false;
   if (precision == 32) return samp_layout<float>(m, true, true).total <= static_cast<size_t>(limit) ||
                               samp_layout<float>(m, true, false).total <= static_cast<size_t>(limit);
-  return samp_layout<double>(m, true, true).total <= static_cast<size_t>(limit);
+  return m.n <= 64 && samp_layout<double>(m, true, true).total <= static_cast<size_t>(limit);
 }
 
 // Plane residency: "shared" keeps a walker's planes in shared memory (one walker per SM
@@ -1186,18 +1094,22 @@ int launch_sample_jpl(const DevModel& m, const DevWalkers& w, int precision, int
       return launch_sample_t<float, JPL, 512, true, false>(m, w, stream);
     return launch_sample_global<float, JPL>(m, w, stream);
   }
-  if (samp_layout<double>(m, true, true).total <= static_cast<size_t>(limit)) {
-    if constexpr (JPL == 1) {
-      // small planes (n ≤ 32): 128 threads per walker (1D L16: 1.95M vs 1.33M sweeps/s
-      // with 512, whose barriers cost more than the work they split); MVMC_B200_SMEM_THREADS
-      // = 64|128|256|512 overrides
-      const char* e = std::getenv("MVMC_B200_SMEM_THREADS");
-      const int nt = e ? std::atoi(e) : 128;
-      if (nt == 64) return launch_sample_t<double, JPL, 64, true, true>(m, w, stream);
-      if (nt == 128) return launch_sample_t<double, JPL, 128, true, true>(m, w, stream);
-      if (nt == 256) return launch_sample_t<double, JPL, 256, true, true>(m, w, stream);
+  // FP64 squares in shared memory: sides up to 64 with more planes than fit as tiles and batch
+  // vectors (wider planes always fit as tiles when they fit as squares)
+  if constexpr (JPL <= 2) {
+    if (samp_layout<double>(m, true, true).total <= static_cast<size_t>(limit)) {
+      if constexpr (JPL == 1) {
+        // small planes (n ≤ 32): 128 threads per walker (1D L16: 1.95M vs 1.33M sweeps/s
+        // with 512, whose barriers cost more than the work they split); MVMC_B200_SMEM_THREADS
+        // = 64|128|256|512 overrides
+        const char* e = std::getenv("MVMC_B200_SMEM_THREADS");
+        const int nt = e ? std::atoi(e) : 128;
+        if (nt == 64) return launch_sample_t<double, JPL, 64, true, true>(m, w, stream);
+        if (nt == 128) return launch_sample_t<double, JPL, 128, true, true>(m, w, stream);
+        if (nt == 256) return launch_sample_t<double, JPL, 256, true, true>(m, w, stream);
+      }
+      return launch_sample_t<double, JPL, 512, true, true>(m, w, stream);
     }
-    return launch_sample_t<double, JPL, 512, true, true>(m, w, stream);
   }
   return launch_sample_global<double, JPL>(m, w, stream);
 }

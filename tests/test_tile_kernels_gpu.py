@@ -1,8 +1,10 @@
-"""The tile-based measurement (planes as 8×8 tiles of the upper triangle) at the edges of its
-range: sides around multiples of 8, 32 and 64, one and several planes, few and many samples."""
+"""The tile-based sampler and measurement (planes as 8×8 tiles of the upper triangle) at the
+edges of their ranges: sides around multiples of 8, 32 and 64, one and several planes, few
+and many samples, every exchange mix."""
 import numpy as np
 import pytest
 
+import oracle_lib as ol
 from mvmc_lib import lattice, mvmc
 
 pytestmark = pytest.mark.gpu
@@ -13,6 +15,30 @@ def inputs(tmp_path, lx, ly, n_up, nmp=1, nsp=1, **kw):
     args = dict(n_up=n_up, nmp=nmp, nsp_gauss_leg=nsp, shifts=shifts, samples=2, warmup=2, interval=3)
     args.update(kw)
     return lattice().write_inputs(str(tmp_path), lx, ly, **args)[:2]
+
+
+@pytest.mark.parametrize("lx,ly,n_up,nmp,nsp,kw", [
+    (4, 1, 1, 1, 1, {}),                       # n = 2: one tile, six of its rows padding
+    (9, 1, 4, 1, 1, {}),                       # n = 8: one full tile
+    (12, 1, 5, 1, 1, dict(ex_path=0)),         # n = 10, hops only (eight proposals a batch)
+    (8, 4, 16, 1, 1, dict(ex_path=2)),         # n = 32, exchanges only: the last side of 128 threads
+    (6, 6, 17, 1, 1, {}),                      # n = 34: the first side of 512 threads
+    (5, 5, 11, 2, 2, {}),                      # four planes: a refresh sweeps a plane per warp
+    (8, 8, 32, 4, 2, dict(sub=(2, 1))),        # n = 64, eight planes
+    (9, 8, 33, 1, 2, {}),                      # n = 66: above the warp sweep
+    (14, 13, 84, 1, 1, dict(interval=1)),      # n = 168
+])
+def test_tile_sampler_reproduces_the_oracle_chains(tmp_path, lx, ly, n_up, nmp, nsp, kw):
+    """Saved configurations, counters and draw counts of three chains equal the oracle's:
+    batches of speculative proposals leave the chain as one proposal after the other."""
+    nl, init = inputs(tmp_path, lx, ly, n_up, nmp, nsp, **kw)
+    _, ref = ol.opt_step1_walkers(nl, 3, seed=11, initial_def=init)
+    eng = mvmc().Engine(nl, initial_def=init, walkers=3, precision=64, seed=11)
+    eng.sample()
+    got = eng.samples()
+    for key in ("ele_idx", "proj_cnt", "counter", "draws"):
+        assert got[key].tolist() == ref[key].tolist(), key
+    assert eng.status() == 0
 
 
 @pytest.mark.parametrize("lx,ly,n_up,nmp,nsp,walkers", [

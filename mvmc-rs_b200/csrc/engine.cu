@@ -413,9 +413,6 @@ void build_context(mvmc_b200_ctx* c, const char* namelist, const char* initial_d
   dm.trans_sgn = c->upload(trans_sgn);
   dm.spgl = c->upload(spgl);
   // Slater-derivative site pairs by orbital (the deterministic O_k)
-  MeasTables& mt = c->mt;
-  std::vector<int2> at;
-  std::vector<int> folded;
   {
     std::vector<std::vector<int>> by_orb(std::max(0, m.n_orb));
     for (int a = 0; a < ns; ++a)
@@ -449,47 +446,27 @@ void build_context(mvmc_b200_ctx* c, const char* namelist, const char* initial_d
       size_t longest = 0;
       for (const auto& v : by_orb) longest = std::max(longest, v.size());
       const bool even = longest * by_orb.size() <= 2 * ent.size();
+      MeasTables& mt = c->mt;
       mt.orb_stride = even ? static_cast<int>(by_orb.size()) : 1;
       mt.orb_len = even ? longest * by_orb.size() : ent.size();
-      folded.assign(static_cast<size_t>(dm.nmp) * mt.orb_len, 0);
-      at.resize(by_orb.size());
+      // one upload for both tables: (first entry, count) of every orbital, then the entries
+      std::vector<int> all(2 * by_orb.size() + static_cast<size_t>(dm.nmp) * mt.orb_len, 0);
+      int* folded = all.data() + 2 * by_orb.size();
       for (size_t k = 0; k < by_orb.size(); ++k) {
-        at[k] = make_int2(even ? static_cast<int>(k) : off[k], static_cast<int>(by_orb[k].size()));
+        const int first = even ? static_cast<int>(k) : off[k];
+        all[2 * k] = first;
+        all[2 * k + 1] = static_cast<int>(by_orb[k].size());
         for (int mp = 0; mp < dm.nmp; ++mp)
           for (size_t e = 0; e < by_orb[k].size(); ++e) {
             const int v = by_orb[k][e];
             const int a = tinv[mp * ns + (v >> 16)], b = tinv[mp * ns + ((v >> 1) & 0x7fff)];
             const int sign = ((v & 1) ? -1 : 1) * trans_sgn[mp * ns + a] * trans_sgn[mp * ns + b];
-            folded[mp * mt.orb_len + at[k].x + e * mt.orb_stride] = (a << 16) | (b << 1) | (sign < 0 ? 1 : 0);
+            folded[mp * mt.orb_len + first + e * mt.orb_stride] = (a << 16) | (b << 1) | (sign < 0 ? 1 : 0);
           }
       }
-    }
-  }
-  {
-    std::vector<std::vector<int2>> by_dst(ns2);
-    for (size_t t = 0; t < tval.size(); ++t) {
-      const int* h = &tterm[4 * t];
-      if (h[1] == h[3] && h[0] != h[2])
-        by_dst[h[0] + h[1] * ns].push_back(make_int2(h[2] + h[3] * ns, static_cast<int>(t)));
-    }
-    std::vector<int> hop_off(1, 0);
-    std::vector<int2> hop;
-    for (const auto& v : by_dst) {
-      hop.insert(hop.end(), v.begin(), v.end());
-      hop_off.push_back(static_cast<int>(hop.size()));
-    }
-    // one upload for the four tables, the pairs first (8-byte aligned)
-    std::vector<int> all;
-    for (const std::vector<int2>* v : {&hop, &at})
-      for (const int2& p : *v) all.insert(all.end(), {p.x, p.y});
-    all.insert(all.end(), hop_off.begin(), hop_off.end());
-    all.insert(all.end(), folded.begin(), folded.end());
-    const int* base = c->upload(all);
-    mt.hop = reinterpret_cast<const int2*>(base);
-    mt.hop_off = base + 2 * (hop.size() + at.size());
-    if (!folded.empty()) {
-      mt.orb_at = mt.hop + hop.size();
-      mt.orb_ent = mt.hop_off + hop_off.size();
+      const int* base = c->upload(all);
+      mt.orb_at = reinterpret_cast<const int2*>(base);
+      mt.orb_ent = base + 2 * by_orb.size();
     }
   }
   dm.tterm = c->upload(tterm);

@@ -66,10 +66,6 @@ struct DevModel {
 
 // Tables of the tile-based measurement, derived from the model's lists.
 struct MeasTables {
-  // Transfer terms c†_{i s} c_{j s}, i ≠ j, by destination slot i + s·ns: hop[hop_off[d] ..
-  // hop_off[d + 1]) = (source slot, term).
-  const int* hop_off = nullptr;
-  const int2* hop = nullptr;
   // Slater-derivative site pairs by orbital with a plane's translation applied: entry e of
   // orbital k on translation mp is orb_ent[mp·orb_len + orb_at[k].x + e·orb_stride],
   // e < orb_at[k].y, packed (a << 16) | (b << 1) | (sign < 0), a and b the untranslated sites.

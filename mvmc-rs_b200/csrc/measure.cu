@@ -616,8 +616,7 @@ __global__ void __launch_bounds__(NT, (kSmemPlane || NT > kMeasThreads ? 1 : 2))
 // A sample's planes are swept one after the other as tiles in shared memory (skewtile.cuh):
 // nothing of the sweep leaves the SM, up to n = 224. NT threads per sample: 64 for n ≤ 64 and
 // many samples, so that several share an SM and hide each other's pivot chains, 512 for the
-// planes that fill an SM. The transfer terms run by destination (one Slater row is gathered for all
-// electrons that may hop there), the Slater derivative per orbital: thread k adds the electron
+// planes that fill an SM. The Slater derivative runs per orbital: thread k adds the electron
 // pairs on orbital k's site pairs in a fixed order, so O rows are bitwise repeatable.
 // Small integers (sites, occupations) are kept as 16 and 8 bits: the n = 224 tiles leave 9 KB.
 struct TriLayout {
@@ -714,31 +713,54 @@ __global__ void __launch_bounds__(NT)
       }
       if (tid == 0) pf[q] = pfv;
       const double wq = m.qpw[q];
-      // transfer terms by destination: −Pf·Σ_k X⁻¹[m][k]·F(dst, k) for every electron m that
-      // may hop there (the moved electron's own entry meets X⁻¹[m][m] = 0)
-      for (int d = warp; d < m.ns2; d += nwarp) {
-        const int e0 = __ldg(mt.hop_off + d), e1 = __ldg(mt.hop_off + d + 1);
-        if (num[d] == 1 || e0 == e1) continue;
-        const double* srow = m.slater + (static_cast<size_t>(q) * m.ns2 + d) * m.ns2;
-        double sv[kLanes];
+      // transfer terms −Pf·Σ_k X⁻¹[m][k]·F(dst, k) (the moved electron's own entry meets
+      // X⁻¹[m][m] = 0): a warp tests 32 terms at once and takes the allowed ones four at a time,
+      // so that four rows' gathers and four sums are in flight
+      const double* slq = m.slater + static_cast<size_t>(q) * m.ns2 * m.ns2;
+      int rk[kLanes];
 #pragma unroll
-        for (int c = 0; c < kLanes; ++c) {
-          const int k = lane + 32 * c;
-          sv[c] = k < n ? __ldg(srow + idx[k] + (k >= ne ? ns : 0)) : 0.0;
+      for (int c = 0; c < kLanes; ++c) {
+        const int k = lane + 32 * c;
+        rk[c] = k < n ? idx[k] + (k >= ne ? ns : 0) : 0;
+      }
+      for (int base = warp * 32; base < m.nterm; base += nwarp * 32) {
+        const int t = base + lane;
+        int dst = 0, mi = 0;
+        bool on = false;
+        if (t < m.nterm) {
+          const int4 h = __ldg(reinterpret_cast<const int4*>(m.tterm) + t);
+          const int src = h.z + h.w * ns;
+          dst = h.x + h.y * ns;
+          on = h.y == h.w && h.x != h.z && num[dst] == 0 && num[src] != 0 && cfg[src] >= 0;
+          mi = on ? cfg[src] + h.w * ne : 0;
         }
-        const int spin = d >= ns ? 1 : 0;
-        for (int e = e0; e < e1; ++e) {
-          const int2 h = __ldg(mt.hop + e);  // source slot, term
-          if (num[h.x] == 0 || cfg[h.x] < 0) continue;
-          const int mi = cfg[h.x] + spin * ne;
-          double r = 0.0;
+        unsigned todo = __ballot_sync(0xffffffffu, on);
+        while (todo) {
+          int j[4], mu[4];
+          const double* row[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {  // the last one again where fewer than four are left
+            j[u] = todo ? __ffs(todo) - 1 : j[u > 0 ? u - 1 : 0];
+            todo &= todo - 1;
+            row[u] = slq + static_cast<size_t>(__shfl_sync(0xffffffffu, dst, j[u])) * m.ns2;
+            mu[u] = __shfl_sync(0xffffffffu, mi, j[u]);
+          }
+          double r[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
           for (int c = 0; c < kLanes; ++c) {
             const int k = lane + 32 * c;
-            if (k < n) r += tri_get(T, nb, mi, k) * sv[c];
+            double sv[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) sv[u] = k < n ? __ldg(row[u] + rk[c]) : 0.0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              if (k < n) r[u] += tri_get(T, nb, mu[u], k) * sv[u];
           }
-          r = warp_sum(r);
-          if (lane == 0) tacc[h.y] += wq * (-r * pfv);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            r[u] = warp_sum(r[u]);
+            if (lane == j[u] && (u == 0 || j[u] != j[u - 1])) tacc[t] += wq * (-r[u] * pfv);
+          }
         }
       }
       // Slater derivative by orbital: electron pairs on its translated site pairs
@@ -749,6 +771,7 @@ __global__ void __launch_bounds__(NT)
       for (int k = tid; k < m.norb; k += nt) {
         const int2 at = __ldg(mt.orb_at + k);  // first entry, count
         double acc = 0.0;
+#pragma unroll 4
         for (int e = 0; e < at.y; ++e) {
           const int ent = __ldg(ents + at.x + static_cast<size_t>(e) * mt.orb_stride);
           const int a = ent >> 16, b = (ent >> 1) & 0x7fff;

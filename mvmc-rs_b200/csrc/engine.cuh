@@ -102,6 +102,7 @@ struct DevWalkers {
   double* drift;              // [W] max |Δ ln|IP|| between the tracked and the refreshed amplitude
   long long* nrefresh;        // [W*2] scheduled (C rule / NRefresh) and guard-triggered refreshes
   double refresh_guard;       // refresh after an accepted move with a plane ratio outside [g, 1/g] (0 off)
+  bool preset = false;        // the walkers' first FP32 planes and Pf are in ws64 and pf (k_planes_tri)
   double* s_inv = nullptr;    // [W*saved*nqp*n*n] FP64 X⁻¹ at each save point (resident measurement), or null
   double* s_pf = nullptr;     // [W*saved*nqp] Pf at each save point
 };

@@ -5,7 +5,7 @@
 // together: their row pairs are formed one after the other from the stored matrix plus the
 // panel's own pending updates, and the matrix takes one rank-2K update per panel as a
 // product of the panel with itself. Same pivot rule (p the smallest unswept index, q the
-// first maximum of |A(p, j)| over unswept j), same status codes, same Pf product.
+// maximum of |A(p, j)| over unswept j, to 2⁻¹²: tri_key), same status codes, same Pf product.
 //
 // With u, v the rows p and q before the step and a = A(p, q), the swept matrix is
 //   A'(i, j) = Z(A)(i, j) + (ṽ_i ũ_j − ũ_i ṽ_j)/a,
@@ -183,9 +183,11 @@ __device__ __forceinline__ unsigned tri_key(double x, int j) {
 // pivot; -1 non-finite). T is taken as complete after the call's first barrier and is
 // complete after the call.
 //
-// A panel is a chain of latencies (row, maximum, partner row, reciprocal), so the row of the
-// next pivot is read and brought up to date (but for the current pivot) beside the partner
-// row, and what the chain does not need (the sign of the permutation) is left to the end.
+// A panel is a chain of latencies (row, maximum, partner row, reciprocal; about 1.1k cycles a
+// pivot at n = 224), so the row of the next pivot is read and brought up to date (but for the
+// current pivot) beside the partner row, and the sign of the permutation is summed per lane
+// and reduced once at the end. n = 224, one plane per SM: 0.22 ms, half of it panels and half
+// updates (1.75 ms as a packed triangle with one rank-2 pass per pivot).
 template <int G, int PG, int CPT>
 __device__ void tri_sweep(double* T, double* pan, unsigned char* red, int n, double& pf_out, int& status_out) {
   constexpr int K = kTilePivots;

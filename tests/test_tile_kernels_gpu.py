@@ -64,3 +64,20 @@ def test_tile_measurement_matches_the_square_planes(tmp_path, monkeypatch, lx, l
     assert eng.status() == 0
     for a, b in zip(rows["tiles"], rows["l2"]):
         assert np.max(np.abs(a - b)) <= 1e-9 * max(1.0, np.max(np.abs(b)))
+
+
+@pytest.mark.parametrize("lx,ly,n_up", [(11, 10, 54), (11, 11, 59), (16, 14, 112)])  # n = 108, 118, 224
+def test_mixed_call_starts_from_the_fp64_planes(tmp_path, lx, ly, n_up):
+    """FP32 walkers too wide for an FP64 sweep beside their planes start every call but the first
+    from planes swept beforehand. A chain leaves its FP64 twin only where an FP32 ratio falls
+    across its threshold, which 4 % of the chains of one plane do within such a run: of 16
+    chains more than four with probability below 1e-3, nearly all if the planes were wrong."""
+    nl, init = inputs(tmp_path, lx, ly, n_up, interval=1, samples=1, tp=-0.2)
+    got = {}
+    for precision in (64, 32):
+        eng = mvmc().Engine(nl, initial_def=init, walkers=16, precision=precision, seed=3)
+        eng.sample()
+        eng.sample()
+        got[precision] = eng.samples()["ele_idx"].reshape(16, -1)
+        assert eng.status() == 0
+    assert np.sum(np.any(got[64] != got[32], axis=1)) <= 4

@@ -868,8 +868,8 @@ __global__ void __launch_bounds__(NT)
 // rounding in its operands (two measurements that agree to 1e-15 gave updates 1e-6 to 1e-3
 // apart), such models are the ones compared with other programs digit by digit, and there the
 // tiles saved a fifth of a measurement of a few per cent of the step. From eight planes of 64 on
-// they halve it (2D 8×8, 4096 samples: 11.1 → 4.9 ms), at n = 224 they quarter it (2048
-// samples: 24.3 → 6.2 ms).
+// they halve it (2D 8×8, 4096 samples: 11.1 → 4.6 ms), at n = 224 they quarter it (2048
+// samples: 24.3 → 6.0 ms).
 // Sides up to 64 take two warps per sample when the samples fill the SMs several times over;
 // fewer samples leave the SMs to the latency of one sample, which eight warps shorten.
 int tri_measure_threads(const DevModel& m, const MeasTables& mt, int nsamples, int limit) {

@@ -862,8 +862,14 @@ __global__ void __launch_bounds__(NT)
   }
 }
 
-// Threads per sample of the tile measurement; 0 where it is not used: the planes do not fit, a
-// translation is not a permutation, or the model is small (up to four planes of side 64).
+struct TriMeasPlan {
+  int threads = 0;  // 0: not applicable
+  bool acc = false;
+  size_t smem = 0;
+};
+
+// Threads per sample of the tile measurement; none where it is not used: the planes do not fit, a
+// translation is not a permutation, or the model is small (below eight planes of side 64).
 // Small models keep the square planes and their digits: the SR-CG amplifies any change of
 // rounding in its operands (two measurements that agree to 1e-15 gave updates 1e-6 to 1e-3
 // apart), such models are the ones compared with other programs digit by digit, and there the
@@ -872,31 +878,37 @@ __global__ void __launch_bounds__(NT)
 // samples: 24.3 → 6.0 ms).
 // Sides up to 64 take two warps per sample when the samples fill the SMs several times over;
 // fewer samples leave the SMs to the latency of one sample, which eight warps shorten.
-int tri_measure_threads(const DevModel& m, const MeasTables& mt, int nsamples, int limit) {
+// The plane sums are in shared memory where they take no more than a quarter of the rest, else in
+// the block's workspace (gws_stride doubles); lists longer than the workspace (dilute models,
+// long-range hopping: more than 2n² terms) need the shared memory. It holds them wherever the
+// square planes' layout, with its two copies, would.
+TriMeasPlan tri_measure_plan(const DevModel& m, const MeasTables& mt, int nsamples, size_t gws_stride, int limit) {
+  TriMeasPlan p;
   const bool small = m.n <= 64 && static_cast<long long>(m.nqp) * m.n * m.n < 8 * 64 * 64;
-  if (small || !mt.orb_ent || m.n > 224 || m.ns2 > 32767 || tri_layout(m, false).total + 512 > static_cast<size_t>(limit))
-    return 0;
+  if (small || !mt.orb_ent || m.n > 224 || m.ns2 > 32767) return p;
+  const size_t plain = tri_layout(m, false).total, with = tri_layout(m, true).total, room = static_cast<size_t>(limit) - 512;
+  const bool in_ws = gws_stride >= static_cast<size_t>(m.nterm);
+  p.acc = with <= room && (!in_ws || with <= plain + plain / 4);
+  p.smem = p.acc ? with : plain;
+  if (p.smem > room || (!p.acc && !in_ws)) return p;
   const bool many = nsamples > 4 * current_device_attr(cudaDevAttrMultiProcessorCount);
-  return m.n <= 64 ? (many ? 64 : 256) : (m.n <= 128 ? 256 : 512);
+  p.threads = m.n <= 64 ? (many ? 64 : 256) : (m.n <= 128 ? 256 : 512);
+  return p;
 }
 
 template <int NT, int PG, int CPT>
-int launch_measure_tri(const DevModel& m, const MeasTables& mt, const int* s_idx, const int* s_cfg, const int* s_num,
-                       const int* s_cnt, int nsamples, double* gws, size_t gws_stride, int gws_blocks, double* ostore,
-                       double* eloc, double* lpsi, int* valid, unsigned* status, cudaStream_t stream, int limit) {
+int launch_measure_tri(const DevModel& m, const MeasTables& mt, const TriMeasPlan& p, const int* s_idx,
+                       const int* s_cfg, const int* s_num, const int* s_cnt, int nsamples, double* gws,
+                       size_t gws_stride, int gws_blocks, double* ostore, double* eloc, double* lpsi, int* valid,
+                       unsigned* status, cudaStream_t stream) {
   auto kernel = k_measure_tri<NT, PG, CPT>;
-  // the plane sums in shared memory where they take no more than a quarter of the rest
-  const size_t plain = tri_layout(m, false).total, with = tri_layout(m, true).total;
-  const int acc = with <= plain + plain / 4 && with + 512 <= static_cast<size_t>(limit) ? 1 : 0;
-  if (!acc && gws_stride < static_cast<size_t>(m.nterm)) return kErrArgument;
-  const size_t smem = acc ? with : plain;
-  MVMCB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  MVMCB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(p.smem)));
   int per = 0;
-  MVMCB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, NT, smem));
+  MVMCB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, NT, p.smem));
   int grid = std::min(nsamples, std::max(1, per) * current_device_attr(cudaDevAttrMultiProcessorCount));
-  if (!acc) grid = std::min(grid, gws_blocks);
-  kernel<<<std::max(1, grid), NT, smem, stream>>>(m, mt, s_idx, s_cfg, s_num, s_cnt, nsamples, acc, gws, gws_stride,
-                                                  ostore, eloc, lpsi, valid, status);
+  if (!p.acc) grid = std::min(grid, gws_blocks);
+  kernel<<<std::max(1, grid), NT, p.smem, stream>>>(m, mt, s_idx, s_cfg, s_num, s_cnt, nsamples, p.acc ? 1 : 0, gws,
+                                                    gws_stride, ostore, eloc, lpsi, valid, status);
   MVMCB_CUDA(cudaGetLastError());
   return kOk;
 }
@@ -1055,10 +1067,11 @@ int launch_measure(const DevModel& m, const MeasTables& mt, const int* s_idx, co
   // keeps square planes, in shared memory or in L2)
   const size_t gws_stride = static_cast<size_t>(2) * n * n;
   const bool l2 = mode && std::strcmp(mode, "l2") == 0;
-  const int nt = gval || l2 ? 0 : tri_measure_threads(m, mt, nsamples, limit);
-#define MVMCB_MEASURE_TRI(NT, PG, C)                                                                                 \
-  launch_measure_tri<NT, PG, C>(m, mt, s_idx, s_cfg, s_num, s_cnt, nsamples, gws, gws_stride, gws_blocks, ostore, eloc, \
-                                lpsi, valid, status, stream, limit)
+  const TriMeasPlan tri = gval || l2 ? TriMeasPlan{} : tri_measure_plan(m, mt, nsamples, gws_stride, limit);
+  const int nt = tri.threads;
+#define MVMCB_MEASURE_TRI(NT, PG, C)                                                                                  \
+  launch_measure_tri<NT, PG, C>(m, mt, tri, s_idx, s_cfg, s_num, s_cnt, nsamples, gws, gws_stride, gws_blocks, ostore, \
+                                eloc, lpsi, valid, status, stream)
   if (nt == 64) return MVMCB_MEASURE_TRI(64, 64, 1);
   if (nt == 256 && n <= 64) return MVMCB_MEASURE_TRI(256, 64, 1);
   if (nt == 256) return MVMCB_MEASURE_TRI(256, 128, 1);

@@ -66,6 +66,42 @@ def test_tile_measurement_matches_the_square_planes(tmp_path, monkeypatch, lx, l
         assert np.max(np.abs(a - b)) <= 1e-9 * max(1.0, np.max(np.abs(b)))
 
 
+def hoppings_within(path, ns, reach):
+    """Rewrite trans.def: every site hops to its `reach` next sites on either side (in the
+    order of the site index), both spins."""
+    lines = []
+    for i in range(ns):
+        for d in range(1, reach + 1):
+            for j in ((i + d) % ns, (i - d) % ns):
+                lines += [f"{i:5d} {s:5d} {j:5d} {s:5d} {0.1 / d: .15f} {0.0: .15f}\n" for s in (0, 1)]
+    lattice()._def_file(str(path / "trans.def"), "NTransfer", len(lines), "".join(lines))
+
+
+@pytest.mark.parametrize("lx,ly,n_up,nmp,nsp,reach,walkers", [
+    (8, 8, 8, 64, 2, 0, 3),     # 1024 terms, n = 16, 128 planes
+    (8, 8, 8, 64, 2, 0, 700),   # the same, two warps per sample
+    (16, 16, 16, 64, 1, 0, 3),  # 4096 terms, n = 32, 64 planes
+    (9, 8, 33, 1, 1, 35, 3),    # 70 of 71 other sites, n = 66: 10080 terms
+])
+def test_more_terms_than_the_workspace_holds(tmp_path, lx, ly, n_up, nmp, nsp, reach, walkers):
+    """More than 2n² transfer terms: the plane sums no longer fit the block's workspace. Energies
+    and O rows of three chains against the oracle's (one plane's condition number, 1e5, times
+    the rounding of its sweep, as above)."""
+    shifts = [(x, y) for y in range(ly) for x in range(lx)]
+    nl, init = inputs(tmp_path, lx, ly, n_up, nmp, nsp, shifts=shifts, interval=1, samples=1, warmup=1, tp=-0.2)
+    if reach:
+        hoppings_within(tmp_path, lx * ly, reach)
+    _, ref = ol.opt_step1_walkers(nl, 3, seed=7, initial_def=init)
+    eng = mvmc().Engine(nl, initial_def=init, walkers=walkers, precision=64, seed=7)
+    eng.sample()
+    assert eng.samples()["ele_idx"].reshape(walkers, -1)[:3].tolist() == ref["ele_idx"].reshape(3, -1).tolist()
+    eng.measure()
+    o = eng.o_store()[:3]
+    assert np.allclose(o, ref["ostore"].reshape(3, -1), rtol=1e-9, atol=1e-9 * np.abs(ref["ostore"]).max())
+    assert abs(eng.local_energies()[:3].mean() - ref["energy"][1]) <= 1e-9 * abs(ref["energy"][1])
+    assert eng.status() == 0
+
+
 @pytest.mark.parametrize("lx,ly,n_up", [(11, 10, 54), (11, 11, 59), (16, 14, 112)])  # n = 108, 118, 224
 def test_mixed_call_starts_from_the_fp64_planes(tmp_path, lx, ly, n_up):
     """FP32 walkers too wide for an FP64 sweep beside their planes start every call but the first

@@ -4,8 +4,8 @@
 // The sweep of pfinv.cuh takes n/2 rank-2 passes over the matrix. Here K pivots are taken
 // together: their row pairs are formed one after the other from the stored matrix plus the
 // panel's own pending updates, and the matrix takes one rank-2K update per panel as a
-// product of the panel with itself. Same pivot rule (p the smallest unswept index, q the
-// maximum of |A(p, j)| over unswept j, to 2⁻¹²: tri_key), same status codes, same Pf product.
+// product of the panel with itself. Same pivot rule (p the smallest unswept index, q the first
+// maximum of |A(p, j)| over unswept j), same status codes, same Pf product.
 //
 // With u, v the rows p and q before the step and a = A(p, q), the swept matrix is
 //   A'(i, j) = Z(A)(i, j) + (ṽ_i ũ_j − ũ_i ṽ_j)/a,
@@ -40,8 +40,9 @@ __host__ __device__ constexpr int tri_pan_stride(int n) { return (n + 15) / 16 *
 __host__ __device__ constexpr size_t tri_pan_doubles(int n) {
   return static_cast<size_t>(2 * kTilePivots) * tri_pan_stride(n);
 }
-// Cross-warp pivot search (one key per warp), the status, the parity and Pf.
-constexpr size_t kTriRedBytes = 16 * 4 + 2 * 4 + 8;
+// Cross-warp pivot search (|x| and column of each panel warp's candidate), the status, the
+// parity and Pf.
+constexpr size_t kTriRedBytes = 8 * 8 + 8 * 4 + 2 * 4 + 8;
 
 __device__ __forceinline__ int tri_tile(int nb, int I, int J) { return I * nb - I * (I + 1) / 2 + J; }
 
@@ -166,14 +167,27 @@ __device__ __forceinline__ void tri_panel_bar() {
   else asm volatile("bar.sync 1, %0;" ::"n"(PG) : "memory");
 }
 
-// Order key of a pivot candidate: 23 leading bits of |x| above the reversed column index, so
-// that one integer maximum finds the largest entry, the lowest column among entries that
-// agree to 2⁻¹². (The pivot is then within 2⁻¹² of the largest: the growth bound of partial
-// pivoting is unchanged to that factor.) 0: not a candidate (zero or NaN).
-__device__ __forceinline__ unsigned tri_key(double x, int j) {
-  const unsigned hi = static_cast<unsigned>(__double2hiint(x)) & 0x7fffffffu;
-  const bool ok = x == x && (hi | static_cast<unsigned>(__double2loint(x))) != 0u;
-  return ok ? (max(hi >> 8, 1u) << 8) | static_cast<unsigned>(255 - j) : 0u;
+// |x| as an integer of the same order; 0 (no pivot) for zero and NaN.
+__device__ __forceinline__ unsigned long long tri_abs(double x) {
+  return x == x ? static_cast<unsigned long long>(__double_as_longlong(x)) & 0x7fffffffffffffffull : 0ull;
+}
+
+// The lane that holds the largest |x| of the warp's candidates (`at`, in column `col`), the
+// lowest column among equal ones; -1 where all are zero. The high words decide unless two
+// agree in them (then the low words, then the columns): one reduction and one vote on the chain.
+__device__ __forceinline__ int tri_warp_max(unsigned long long at, int col) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const unsigned hi = static_cast<unsigned>(at >> 32), lo = static_cast<unsigned>(at);
+  const unsigned top = __reduce_max_sync(kAll, hi);
+  unsigned who = __ballot_sync(kAll, hi == top);
+  if (who & (who - 1)) {
+    const unsigned low = __reduce_max_sync(kAll, hi == top ? lo : 0u);
+    if ((top | low) == 0u) return -1;
+    const bool mine = hi == top && lo == low;
+    const unsigned first = __reduce_min_sync(kAll, mine ? static_cast<unsigned>(col) : kAll);
+    who = __ballot_sync(kAll, mine && static_cast<unsigned>(col) == first);
+  }
+  return __ffs(static_cast<int>(who)) - 1;
 }
 
 // Sweep of the n×n skew matrix in T by G threads (a warp, or the whole block; every thread
@@ -194,8 +208,9 @@ __device__ void tri_sweep(double* T, double* pan, unsigned char* red, int n, dou
   const int tg = G == 32 ? (threadIdx.x & 31) : threadIdx.x;
   const int lane = tg & 31, warp = tg >> 5;
   const int nb = tri_blocks(n), ps = tri_pan_stride(n);
-  unsigned* rkey = reinterpret_cast<unsigned*>(red);
-  int* rint = reinterpret_cast<int*>(red + 64);
+  unsigned long long* rabs = reinterpret_cast<unsigned long long*>(red);
+  int* rcol = reinterpret_cast<int*>(red + 64);
+  int* rint = reinterpret_cast<int*>(red + 96);
   for (int j = tg; j < 2 * K * ps; j += G) pan[j] = 0.0;  // the padding stays zero
   if (tg == 0) rint[0] = 0;
   const bool panel = tg < PG;
@@ -254,26 +269,36 @@ __device__ void tri_sweep(double* T, double* pan, unsigned char* red, int n, dou
 #pragma unroll
           for (int c = 0; c < CPT; ++c) x[c] = fma(vp, u[k - 1][c], fma(-up, v[k - 1][c], x[c]));
         }
-        unsigned key = 0;
+        unsigned long long big = 0ull;
+        int q = n;
 #pragma unroll
         for (int c = 0; c < CPT; ++c) {
           const int j = tg + PG * c;
-          if (!((own >> c) & 1u) && j != p) key = max(key, tri_key(x[c], j));
+          const unsigned long long v = tri_abs(x[c]);
+          if (!((own >> c) & 1u) && j != p && v > big) {
+            big = v;
+            q = j;
+          }
           if (j < n) pan[2 * k * ps + j] = x[c];
         }
-        key = __reduce_max_sync(0xffffffffu, key);
+        int src = tri_warp_max(big, q);
         if constexpr (PG == 32) {
           __syncwarp();
         } else {
-          if (lane == 0) rkey[warp] = key;
+          if (lane == max(src, 0)) {
+            rabs[warp] = big;
+            rcol[warp] = q;
+          }
           tri_panel_bar<G, PG>();
-          key = __reduce_max_sync(0xffffffffu, lane < PG / 32 ? rkey[lane] : 0u);
+          big = lane < PG / 32 ? rabs[lane] : 0ull;
+          q = lane < PG / 32 ? rcol[lane] : n;
+          src = tri_warp_max(big, q);
         }
-        if (key == 0u) {  // no pivot: every thread of the panel sees it
+        if (src < 0) {  // no pivot: every thread of the panel sees it
           status = p + 1;
           break;
         }
-        const int q = 255 - static_cast<int>(key & 255u);
+        q = __shfl_sync(0xffffffffu, q, src);
         const double a = pan[2 * k * ps + q];
         if (lane == (p >> 5)) swept |= 1u << (p & 31);
         if (lane == (q >> 5)) swept |= 1u << (q & 31);
@@ -348,7 +373,7 @@ __device__ void tri_sweep(double* T, double* pan, unsigned char* red, int n, dou
   status = rint[0];
   tri_bar<G>();  // the matrix is complete
   // sgn(σ) and Pf from the panel's first warp
-  double* rpf = reinterpret_cast<double*>(red + 72);
+  double* rpf = reinterpret_cast<double*>(red + 104);
   if (tg < 32) {
     passed = __reduce_add_sync(0xffffffffu, passed);
     if (tg == 0) {

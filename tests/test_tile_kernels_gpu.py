@@ -66,6 +66,33 @@ def test_tile_measurement_matches_the_square_planes(tmp_path, monkeypatch, lx, l
         assert np.max(np.abs(a - b)) <= 1e-9 * max(1.0, np.max(np.abs(b)))
 
 
+@pytest.mark.parametrize("sites,walkers", [
+    (2, 64),     # n = 4, a warp per plane, a column per lane
+    (18, 450),   # n = 36, two columns per lane
+    (34, 64),    # n = 68, eight warps per panel
+    (34, 160),   # four warps per panel
+])
+def test_pivot_is_the_largest_entry(tmp_path, monkeypatch, sites, walkers):
+    """Planes of 2×2 blocks ((x, v), (b, 0)), v = x + 2⁻²⁰, in each walker's own electron order. The
+    inverse has a zero where x stands, which the sweep keeps exactly with v as pivot; with x,
+    where it comes first, it becomes the rounding of 1/x − v·(1/x)·(1/v). Sites are full and
+    only exchanges are tried, so no move is made and the resident measurement shows the
+    sampler's sweep."""
+    nl, init = inputs(tmp_path, sites, 1, sites, sub=(sites, 1), ex_path=2, interval=1, samples=1, warmup=1)
+    for mode, resident in (("l2", 0), ("tiles", 0), ("tiles", 1)):
+        monkeypatch.setenv("MVMC_B200_MEASURE", mode)
+        eng = mvmc().Engine(nl, initial_def=init, walkers=walkers, precision=64, seed=5, measure_resident=resident)
+        p = np.zeros(eng.dims["npara"])
+        f = p[eng.dims["nproj"]:].reshape(sites, sites)  # [site, displacement]
+        f[0::2, 0], f[0::2, 1], f[1::2, sites - 1] = 0.9, 0.9 + 2.0 ** -20, 0.6
+        eng.set_parameters(p)
+        eng.sample()
+        eng.measure()
+        assert eng.status() == 0
+        o = eng.o_store()[:, 1 + eng.dims["nproj"]:].reshape(walkers, sites, sites)
+        assert np.all(o[:, 0::2, 1] != 0.0) and np.all(o[:, 0::2, 0] == 0.0), (mode, resident)
+
+
 def hoppings_within(path, ns, reach):
     """Rewrite trans.def: every site hops to its `reach` next sites on either side (in the
     order of the site index), both spins."""

@@ -869,13 +869,17 @@ struct TriMeasPlan {
 };
 
 // Threads per sample of the tile measurement; none where it is not used: the planes do not fit, a
-// translation is not a permutation, or the model is small (below eight planes of side 64).
-// Small models keep the square planes and their digits: the SR-CG amplifies any change of
-// rounding in its operands (two measurements that agree to 1e-15 gave updates 1e-6 to 1e-3
-// apart), such models are the ones compared with other programs digit by digit, and there the
-// tiles saved a fifth of a measurement of a few per cent of the step. From eight planes of 64 on
-// they halve it (2D 8×8, 4096 samples: 11.1 → 4.6 ms), at n = 224 they quarter it (2048
-// samples: 24.3 → 6.0 ms).
+// translation is not a permutation, or the square planes are kept for one of two reasons.
+//  - Up to four planes of side 64: their digits. The SR-CG amplifies any change of rounding in
+//    its operands (two measurements that agree to 1e-15 gave updates 1e-6 to 1e-3 apart), and
+//    whole optimisation steps of such models are compared with earlier ones more tightly. It
+//    costs them up to 0.6 of the measurement (4096 samples, squares and tiles: one plane of 16
+//    0.57 and 0.47 ms, of 32 0.84 and 0.63, of 64 2.10 and 0.99; four of 64 6.17 and 2.52).
+//  - Sides up to 32 with samples for at most four blocks per SM: time (32 planes of 32, 300
+//    samples: 1.7 ms in squares, 2.8 on tiles; 600 samples: 3.1 and 2.5).
+// Elsewhere the tiles are faster (4096 samples: eight planes of 16 1.47 and 1.00 ms, of 32 3.2 and
+// 2.0, of 48 8.1 and 2.8, of 64 11.7 and 4.7; 148 samples, eight planes of 34 0.50 and 0.46;
+// n = 224, 2048 samples, 24.3 and 6.1).
 // Sides up to 64 take two warps per sample when the samples fill the SMs several times over;
 // fewer samples leave the SMs to the latency of one sample, which eight warps shorten.
 // The plane sums are in shared memory where they take no more than a quarter of the rest, else in
@@ -884,14 +888,14 @@ struct TriMeasPlan {
 // square planes' layout, with its two copies, would.
 TriMeasPlan tri_measure_plan(const DevModel& m, const MeasTables& mt, int nsamples, size_t gws_stride, int limit) {
   TriMeasPlan p;
-  const bool small = m.n <= 64 && static_cast<long long>(m.nqp) * m.n * m.n < 8 * 64 * 64;
-  if (small || !mt.orb_ent || m.n > 224 || m.ns2 > 32767) return p;
+  const bool many = nsamples > 4 * current_device_attr(cudaDevAttrMultiProcessorCount);
+  const bool squares = (m.n <= 64 && m.nqp <= 4) || (m.n <= 32 && !many);
+  if (squares || !mt.orb_ent || m.n > 224 || m.ns2 > 32767) return p;
   const size_t plain = tri_layout(m, false).total, with = tri_layout(m, true).total, room = static_cast<size_t>(limit) - 512;
   const bool in_ws = gws_stride >= static_cast<size_t>(m.nterm);
   p.acc = with <= room && (!in_ws || with <= plain + plain / 4);
   p.smem = p.acc ? with : plain;
   if (p.smem > room || (!p.acc && !in_ws)) return p;
-  const bool many = nsamples > 4 * current_device_attr(cudaDevAttrMultiProcessorCount);
   p.threads = m.n <= 64 ? (many ? 64 : 256) : (m.n <= 128 ? 256 : 512);
   return p;
 }

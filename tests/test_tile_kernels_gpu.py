@@ -44,6 +44,10 @@ def test_tile_sampler_reproduces_the_oracle_chains(tmp_path, lx, ly, n_up, nmp, 
 @pytest.mark.parametrize("lx,ly,n_up,nmp,nsp,walkers", [
     (8, 8, 32, 4, 2, 700),     # n = 64, eight planes: two warps per sample
     (8, 8, 32, 4, 2, 40),      # the same, eight warps per sample
+    (8, 8, 31, 4, 2, 700),     # n = 62
+    (7, 5, 17, 4, 2, 40),      # n = 34
+    (8, 4, 16, 4, 2, 700),     # n = 32
+    (8, 4, 4, 4, 2, 700),      # n = 8: one tile
     (9, 8, 33, 1, 2, 9),       # n = 66, 256 threads
     (11, 12, 64, 1, 1, 9),     # n = 128
     (11, 12, 65, 1, 1, 9),     # n = 130, 512 threads
@@ -91,6 +95,24 @@ def test_pivot_is_the_largest_entry(tmp_path, monkeypatch, sites, walkers):
         assert eng.status() == 0
         o = eng.o_store()[:, 1 + eng.dims["nproj"]:].reshape(walkers, sites, sites)
         assert np.all(o[:, 0::2, 1] != 0.0) and np.all(o[:, 0::2, 0] == 0.0), (mode, resident)
+
+
+@pytest.mark.parametrize("lx,ly,n_up,nmp,nsp,walkers", [
+    (8, 8, 32, 4, 1, 700),     # n = 64, four planes: the digits of the square planes
+    (8, 4, 16, 16, 2, 40),     # n = 32, 32 planes, few samples: the squares are faster
+])
+def test_measurement_on_square_planes_beside_the_tiles(tmp_path, monkeypatch, lx, ly, n_up, nmp, nsp, walkers):
+    """Where the choice falls on the square planes the results are theirs bit for bit."""
+    shifts = [(x, y) for y in range(ly) for x in range(lx)]
+    nl, init = inputs(tmp_path, lx, ly, n_up, nmp, nsp, shifts=shifts, interval=1, samples=1)
+    eng = mvmc().Engine(nl, initial_def=init, walkers=walkers, precision=64, seed=5)
+    eng.sample()
+    rows = []
+    for mode in ("tiles", "l2"):
+        monkeypatch.setenv("MVMC_B200_MEASURE", mode)
+        eng.measure()
+        rows.append(eng.o_store())
+    assert np.array_equal(*rows)
 
 
 def hoppings_within(path, ns, reach):

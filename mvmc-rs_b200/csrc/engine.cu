@@ -23,6 +23,7 @@ int launch_sample(const DevModel& m, const DevWalkers& w, int precision, cudaStr
 bool sample_planes_in_smem(const DevModel& m, int precision, int limit);
 bool sample_tri_applies(const DevModel& m, int precision, int limit);
 int launch_sample_tri(const DevModel& m, const DevWalkers& w, int precision, int limit, cudaStream_t stream);
+bool measure_on_squares(const DevModel& m, int nsamples);
 int launch_measure(const DevModel& m, const MeasTables& mt, const int* s_idx, const int* s_cfg, const int* s_num,
                    const int* s_cnt, int nsamples, double* gws, int gws_blocks, double* ostore,
                    double* eloc, double* lpsi, int* valid, double* gval, unsigned* status, cudaStream_t stream);
@@ -441,8 +442,10 @@ void build_context(mvmc_b200_ctx* c, const char* namelist, const char* initial_d
       dm.orb_off = c->upload(off);
       dm.orb_ent = c->upload(ent);
       dm.trans_inv = c->upload(tinv);
-      // the same pairs per translation, signs folded in; interleaved over the orbitals unless
-      // padding to the longest list would more than double the table
+    }
+    // For the tile measurement the same pairs per translation, signs folded in; interleaved over
+    // the orbitals unless padding to the longest list would more than double the table.
+    if (dm.orb_off && !opt.c_order && !measure_on_squares(dm, c->W * c->S)) {
       size_t longest = 0;
       for (const auto& v : by_orb) longest = std::max(longest, v.size());
       const bool even = longest * by_orb.size() <= 2 * ent.size();

@@ -862,14 +862,11 @@ __global__ void __launch_bounds__(NT)
   }
 }
 
-struct TriMeasPlan {
-  int threads = 0;  // 0: not applicable
-  bool acc = false;
-  size_t smem = 0;
-};
+// More samples than four blocks per SM take at a time.
+bool many_samples(int nsamples) { return nsamples > 4 * current_device_attr(cudaDevAttrMultiProcessorCount); }
 
-// Threads per sample of the tile measurement; none where it is not used: the planes do not fit, a
-// translation is not a permutation, or the square planes are kept for one of two reasons.
+// Models that the tile measurement does not take, whatever else: planes too large, sites beyond 16
+// bits, and those whose square planes are kept for one of two reasons.
 //  - Up to four planes of side 64: their digits. The SR-CG amplifies any change of rounding in
 //    its operands (two measurements that agree to 1e-15 gave updates 1e-6 to 1e-3 apart), and
 //    whole optimisation steps of such models are compared with earlier ones more tightly. It
@@ -880,6 +877,18 @@ struct TriMeasPlan {
 // Elsewhere the tiles are faster (4096 samples: eight planes of 16 1.47 and 1.00 ms, of 32 3.2 and
 // 2.0, of 48 8.1 and 2.8, of 64 11.7 and 4.7; 148 samples, eight planes of 34 0.50 and 0.46;
 // n = 224, 2048 samples, 24.3 and 6.1).
+bool measure_on_squares(const DevModel& m, int nsamples) {
+  return m.n > 224 || m.ns2 > 32767 || (m.n <= 64 && m.nqp <= 4) || (m.n <= 32 && !many_samples(nsamples));
+}
+
+struct TriMeasPlan {
+  int threads = 0;  // 0: not applicable
+  bool acc = false;
+  size_t smem = 0;
+};
+
+// Threads per sample of the tile measurement; none where it is not used (also: the planes do not
+// fit beside the lists, or a translation is not a permutation).
 // Sides up to 64 take two warps per sample when the samples fill the SMs several times over;
 // fewer samples leave the SMs to the latency of one sample, which eight warps shorten.
 // The plane sums are in shared memory where they take no more than a quarter of the rest, else in
@@ -888,15 +897,13 @@ struct TriMeasPlan {
 // square planes' layout, with its two copies, would.
 TriMeasPlan tri_measure_plan(const DevModel& m, const MeasTables& mt, int nsamples, size_t gws_stride, int limit) {
   TriMeasPlan p;
-  const bool many = nsamples > 4 * current_device_attr(cudaDevAttrMultiProcessorCount);
-  const bool squares = (m.n <= 64 && m.nqp <= 4) || (m.n <= 32 && !many);
-  if (squares || !mt.orb_ent || m.n > 224 || m.ns2 > 32767) return p;
+  if (!mt.orb_ent || measure_on_squares(m, nsamples)) return p;
   const size_t plain = tri_layout(m, false).total, with = tri_layout(m, true).total, room = static_cast<size_t>(limit) - 512;
   const bool in_ws = gws_stride >= static_cast<size_t>(m.nterm);
   p.acc = with <= room && (!in_ws || with <= plain + plain / 4);
   p.smem = p.acc ? with : plain;
   if (p.smem > room || (!p.acc && !in_ws)) return p;
-  p.threads = m.n <= 64 ? (many ? 64 : 256) : (m.n <= 128 ? 256 : 512);
+  p.threads = m.n <= 64 ? (many_samples(nsamples) ? 64 : 256) : (m.n <= 128 ? 256 : 512);
   return p;
 }
 

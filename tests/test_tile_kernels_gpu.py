@@ -1,6 +1,10 @@
 """The tile-based sampler and measurement (planes as 8×8 tiles of the upper triangle) at the
 edges of their ranges: sides around multiples of 8, 32 and 64, one and several planes, few
-and many samples, every exchange mix."""
+and many samples, every exchange mix; and the square-plane sampler on the models left to it."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -39,6 +43,67 @@ def test_tile_sampler_reproduces_the_oracle_chains(tmp_path, lx, ly, n_up, nmp, 
     for key in ("ele_idx", "proj_cnt", "counter", "draws"):
         assert got[key].tolist() == ref[key].tolist(), key
     assert eng.status() == 0
+
+
+@pytest.mark.parametrize("lx,ly,n_up,nmp,nsp,walkers", [
+    (6, 6, 17, 1, 1, 160),     # n = 34: 256 threads, the block sweeps
+    (8, 4, 16, 4, 1, 160),     # n = 32, four planes: 256 threads, a plane per warp
+    (8, 8, 32, 4, 1, 160),     # n = 64
+    (9, 8, 33, 1, 1, 160),     # n = 66
+    (16, 8, 64, 1, 1, 160),    # n = 128: the last side of 256 threads
+    (8, 4, 16, 4, 1, 460),     # n = 32: 128 threads, a column per lane
+    (6, 6, 17, 1, 1, 460),     # n = 34: 128 threads, two columns per lane
+    (8, 8, 32, 1, 2, 460),     # n = 64
+])
+def test_tile_sampler_with_several_walkers_per_sm(tmp_path, lx, ly, n_up, nmp, nsp, walkers):
+    """More walkers than SMs take 256 or 128 threads each. A chain depends on its seed alone:
+    the first three equal the oracle's."""
+    nl, init = inputs(tmp_path, lx, ly, n_up, nmp, nsp)
+    _, ref = ol.opt_step1_walkers(nl, 3, seed=11, initial_def=init)
+    eng = mvmc().Engine(nl, initial_def=init, walkers=walkers, precision=64, seed=11)
+    eng.sample()
+    got = eng.samples()
+    for key in ("ele_idx", "proj_cnt", "counter", "draws"):
+        assert got[key].reshape(walkers, -1)[:3].ravel().tolist() == ref[key].tolist(), key
+    assert eng.status() == 0
+
+
+SQUARE_PLANES = [
+    (16, 1, 8, 16, 4, "auto"),    # n = 16, 64 planes: squares in shared memory, 128 threads
+    (6, 6, 17, 18, 1, "auto"),    # n = 34, 18 planes: squares, 512 threads
+    (8, 8, 32, 16, 1, "auto"),    # n = 64, 16 planes: planes in L2
+    (16, 16, 113, 1, 1, "auto"),  # n = 226: the first side without tiles
+    (16, 16, 128, 1, 1, "auto"),  # n = 256: the half-filled lattice
+    (8, 8, 32, 4, 2, "global"),   # planes in L2 on request
+    (11, 10, 54, 1, 1, "global"),
+]
+
+
+def square_plane_chains(path, lx, ly, n_up, nmp, nsp):
+    shifts = [(x, y) for y in range(ly) for x in range(lx)]
+    nl, init, _ = lattice().write_inputs(path, lx, ly, n_up=n_up, nmp=nmp, nsp_gauss_leg=nsp, shifts=shifts, samples=2,
+                                         warmup=2, interval=2)
+    _, ref = ol.opt_step1_walkers(nl, 3, seed=11, initial_def=init)
+    eng = mvmc().Engine(nl, initial_def=init, walkers=3, precision=64, seed=11)
+    eng.sample()
+    got = eng.samples()
+    for key in ("ele_idx", "proj_cnt", "counter", "draws"):
+        assert got[key].tolist() == ref[key].tolist(), key
+    e = eng.measure()[0]
+    assert np.allclose(e, ref["energy"], rtol=1e-9)
+    assert eng.status() == 0
+
+
+@pytest.mark.parametrize("lx,ly,n_up,nmp,nsp,residency", SQUARE_PLANES)
+def test_square_plane_sampler_reproduces_the_oracle_chains(tmp_path, lx, ly, n_up, nmp, nsp, residency):
+    """FP64 models whose planes do not fit as tiles, or are asked to stay in L2, run on square
+    planes. In a process of its own: the residency is read once."""
+    code = ("import test_tile_kernels_gpu as t; "
+            f"t.square_plane_chains({str(tmp_path)!r}, {lx}, {ly}, {n_up}, {nmp}, {nsp})")
+    env = dict(os.environ, MVMC_B200_RESIDENCY=residency)
+    run = subprocess.run([sys.executable, "-c", code], cwd=os.path.dirname(os.path.abspath(__file__)), env=env,
+                         capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stderr[-2000:]
 
 
 @pytest.mark.parametrize("lx,ly,n_up,nmp,nsp,walkers", [

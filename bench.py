@@ -43,10 +43,6 @@ sys.path.insert(0, os.path.join(ROOT, "mvmc-rs_b200"))
 WALKERS = {"chain16": 256, "square8": 4096, "square16": 2048, "square16_sr": 8192}
 PFINV = {"pfinv64": [64] * 8192, "pfinv_mix": [32, 48, 64, 96, 128] * 1638}
 METRIC = "Metropolis sweeps/s & SR-step time: mixed vs FP64 path on 1 B200 at |dE|/N<=1e-6"
-# DRAM bytes (read + write) per walker-sweep of k_sample_tri from an ncu capture of a small
-# case of the same kernel instance (profiles/k_sample_tri_square8_w148.txt: 1.905 MB over
-# 148 walkers x 5 sweeps), scaled to a launch by walker-sweeps.
-SAMPLE_DRAM_PER_WALKER_SWEEP = {("square8", 64): 1.905e6 / (148 * 5)}
 PFINV_METRIC = "Pfaffian+inverse/s (batched skew FP64)"
 PHYSCAL = {"physcal8": 4096}
 PHYSCAL_METRIC = "PhysCal samples/s (energy + one- and two-body Green functions, FP64)"
@@ -301,12 +297,23 @@ def time_engine(args, precision, W, namelist, initial_def, cfg, dims, rank, loca
     else:
         t_wall_ms = t_wall * 1e3
     samples = eng.samples()
-    c = samples["counter"].reshape(-1, 6).sum(axis=0)
+    c = samples["counter"].reshape(-1, 6).sum(axis=0)  # of the last block
     drift = eng.refresh_stats()
     eng.close()
     return {"ms": ms, "t_wall_ms": t_wall_ms, "sample_ms": sum(samp) / len(samp),
             "measure_ms": sum(meas) / len(meas), "h2d": h1 - h0, "d2h": d1 - d0, "energy": energy,
-            "acceptance": (c[1] + c[3]) / max(1, c[0] + c[2]), "cg_iters": cg_iters, "drift": drift}
+            "acceptance": (c[1] + c[3]) / max(1, c[0] + c[2]), "cg_iters": cg_iters, "drift": drift,
+            "moves": [int(v) for v in c[:4]]}
+
+
+def sample_flops(dims, walkers, moves, refreshes):
+    """FP64 flops that one block's proposals and refreshes cannot do without, over all walkers:
+    a proposed hop one row of X·v, a proposed exchange X·v, an accepted move the other product
+    and the rank-2 or rank-4 update of one triangle, a refresh the sweep of one triangle (n³)."""
+    n, nqp = dims["n"], dims["nqp"]
+    hops, hops_taken, swaps, swaps_taken = moves
+    per_plane = 2.0 * n * hops + 2.0 * n * n * swaps + 4.0 * n * n * hops_taken + 6.0 * n * n * swaps_taken
+    return nqp * (per_plane + walkers * refreshes * float(n) ** 3)
 
 
 def accuracy_check(args, W, namelist, initial_def, local):
@@ -545,16 +552,27 @@ def engine_bench(args, ws, rank, local):
     sweeps_total = ws * W * sweeps_per_walker_step * args.steps
     value = sweeps_total / (main_rec["ms"] / 1e3)
     n, nqp, ns = dims["n"], dims["nqp"], dims["nsite"]
-    s_bytes = 8 if args.precision == 64 else 4
     p_acc = main_rec["acceptance"]
-    # algorithmic bytes per walker-sweep of the resident sampler (InvM row + gathered Slater
-    # row per proposal, rank-2 read+write per accepted move)
-    per_sweep = ns * (nqp * n * s_bytes + nqp * n * 8) + ns * p_acc * nqp * (2 * n * n * s_bytes)
-    launch_bytes = W * sweeps_per_walker_step * per_sweep
-    achieved = launch_bytes / (main_rec["sample_ms"] / 1e3) / 1e9
-    per_ws = SAMPLE_DRAM_PER_WALKER_SWEEP.get((args.config, args.precision))
-    traffic = per_ws * W * sweeps_per_walker_step if per_ws and not args.interval else None
-    peak, peak_kind = measured_peaks()
+    sample_s = main_rec["sample_ms"] / 1e3
+    if args.precision == 64 and os.environ.get("MVMC_B200_RESIDENCY") != "global":
+        # every model of this benchmark fits as tiles in shared memory: nothing of the planes
+        # moves through L2 or HBM, so the rate is that of the FP64 pipe
+        flops = sample_flops(dims, W, main_rec["moves"], main_rec["drift"]["refreshes"])
+        achieved, peak = flops / sample_s / 1e12, fp64_gemm_peak()
+        roofline = {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
+                    "traffic": None, "kernel": "k_sample_tri",
+                    "peak_kind": "measured cuBLAS FP64 GEMM on this GPU", "algorithmic_flops_per_launch": flops}
+    else:
+        # square planes: algorithmic bytes per walker-sweep (a row of the inverse and a gathered
+        # Slater row per proposal, the rank-2 update's read and write per accepted move)
+        s_bytes = 8 if args.precision == 64 else 4
+        per_sweep = ns * (nqp * n * s_bytes + nqp * n * 8) + ns * p_acc * nqp * (2 * n * n * s_bytes)
+        launch_bytes = W * sweeps_per_walker_step * per_sweep
+        achieved = launch_bytes / sample_s / 1e9
+        peak, peak_kind = measured_peaks()
+        roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+                    "traffic": None, "kernel": "k_sample", "peak_kind": peak_kind,
+                    "algorithmic_bytes_per_launch": launch_bytes}
     if rank != 0:
         if ws > 1:
             dist.destroy_process_group()
@@ -579,9 +597,7 @@ def engine_bench(args, ws, rank, local):
         "sr_step_ms": main_rec["ms"] / args.steps, "sample_ms": main_rec["sample_ms"],
         "measure_ms": main_rec["measure_ms"], "energy": main_rec["energy"], "acceptance": p_acc,
         "cg_iterations": main_rec["cg_iters"],
-        "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": achieved / peak, "traffic": traffic, "kernel": "k_sample_tri" if args.precision == 64 else "k_sample",
-                     "peak_kind": peak_kind, "algorithmic_bytes_per_launch": launch_bytes},
+        "roofline": roofline,
         "cpu_baseline": {"value": base_sweeps / base_t, "unit": "sweeps/s", "cores": 1, "kind": "port",
                          "sample": f"1 chain x one SR step (warm-up + {S} blocks, {base_sweeps} sweeps) "
                                    f"of {args.config}"},
@@ -611,14 +627,15 @@ def engine_bench(args, ws, rank, local):
     if os.environ.get("MVMC_B200_TIMERS") == "1":
         out["timers"] = "phase cycles: run the engine directly for mvmc_b200_sampler_timers"
     if not args.no_extra and args.config == "square8" and ws == 1:
-        # the sampler's planes are served from L2: its effective bandwidth against a measured
-        # L2-resident copy as well as against HBM
-        l2 = l2_ceiling_gbs()
-        out["roofline"]["l2_peak"] = max(l2.values())
-        out["roofline"]["l2_frac"] = achieved / max(l2.values())
-        out["roofline"]["l2_peak_kind"] = (
-            "measured in this run: max of a 24 MB -> 24 MB copy (%.0f GB/s) and one reduction "
-            "reading a 24 MB buffer 64 times (%.0f GB/s)" % (l2["copy"], l2["read"]))
+        if roofline["kernel"] == "k_sample":
+            # square planes of this model are served from L2: the effective bandwidth against a
+            # measured L2-resident copy as well as against HBM
+            l2 = l2_ceiling_gbs()
+            roofline["l2_peak"] = max(l2.values())
+            roofline["l2_frac"] = roofline["achieved"] / max(l2.values())
+            roofline["l2_peak_kind"] = (
+                "measured in this run: max of a 24 MB -> 24 MB copy (%.0f GB/s) and one reduction "
+                "reading a 24 MB buffer 64 times (%.0f GB/s)" % (l2["copy"], l2["read"]))
         out["square16_sr"] = sr16_record(args, local)
         out["pfinv"] = pfinv_records(local)
     print(json.dumps(out), flush=True)

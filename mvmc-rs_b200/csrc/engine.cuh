@@ -70,7 +70,8 @@ struct MeasTables {
   // orbital k on translation mp is orb_ent[mp·orb_len + orb_at[k].x + e·orb_stride],
   // e < orb_at[k].y, packed (a << 16) | (b << 1) | (sign < 0), a and b the untranslated sites.
   // Orbitals with about equally many pairs are interleaved (orb_stride = norb), so that a
-  // warp's threads read neighbouring entries. Null: a translation is not a permutation.
+  // warp's threads read neighbouring entries. Null: a translation is not a permutation, or the
+  // model's measurement never runs on tiles.
   const int2* orb_at = nullptr;
   const int* orb_ent = nullptr;
   size_t orb_len = 0;

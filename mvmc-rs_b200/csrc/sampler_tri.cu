@@ -1,8 +1,10 @@
 // K2t: the FP64 sampler with every plane of a walker in shared memory as tiles of the upper
 // triangle, several proposals evaluated per pass (one CTA per walker).
 //
-// The chain is the one of k_sample (sampler.cu): the same draws, moves, decisions and refresh
-// rule. Two things differ.
+// The draws, moves, decision rule and refresh rule are those of k_sample (sampler_impl.cuh).
+// Sums run in another order, so that at a near-singular plane, where an FP64 log-weight is off
+// by up to order 1 in any order, a chain may part from k_sample's (2D 8×8, eight planes: about
+// one decision in 10⁷; neither is nearer to a long-double chain). Two things differ.
 //
 // Storage. A skew plane needs its upper triangle only, so planes that as squares live in L2
 // (2D 8×8 with eight planes of 64: 256 KB; 2D 16×16, n = 224: 401 KB) fit one SM as tiles
@@ -24,7 +26,7 @@
 // Bound by the latency of a batch's phases (2D 8×8, eight planes, one walker per SM: about 15k
 // cycles of vectors and products, 5k of decisions, 11k of update per acceptance, for 2.4
 // proposals). Sampling and measurement against k_sample with its planes in L2: 2D 8×8, 1024
-// walkers, 68.7 → 44.4 ms; 2D 16×16, 1024 walkers, 60.3 → 23.5 ms; a step of the chain of 16
+// walkers, 68.7 → 44.7 ms; 2D 16×16, 1024 walkers, 60.3 → 23.3 ms; a step of the chain of 16
 // sites with 256 walkers, 2.39 → 1.95 ms.
 #include <cuda_runtime.h>
 
@@ -297,7 +299,7 @@ __device__ int draw_window(const DevModel& m, const FastMod& by_ne, const FastMo
 }
 
 // Δ ln P of a hop slot by one warp, from the configuration before the move
-// (log_proj_ratio_hop_warp of sampler.cu, whose occupations are those after it).
+// (log_proj_ratio_hop_warp of sampler_impl.cuh, whose occupations are those after it).
 __device__ double hop_dproj(const DevModel& m, const int* num, const Slot& s) {
   const int lane = threadIdx.x & 31, ns = m.ns, src = s.ri, dst = s.rj;
   double z = 0.0;

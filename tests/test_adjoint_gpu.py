@@ -29,8 +29,8 @@ def inputs(tmp_path, name, interval, **over):
 def test_o_rows_match_central_differences(tmp_path, name, over):
     """64 random (sample, parameter) pairs per model: 2D 8x8 at half filling, 2D 8x8 with
     t' = -0.2 at 56 electrons, and the 2D 16x16 adjoint-check model (t' = -0.2, U = 6,
-    112 + 112 electrons, n = 224, full translation symmetry: inverse planes swept as packed
-    triangles in shared memory)."""
+    112 + 112 electrons, n = 224, full translation symmetry: planes swept as tiles of the upper
+    triangle in shared memory)."""
     nl, init, dims = inputs(tmp_path, name, 2, **over)
     W = 32
     eng = mvmc().Engine(nl, init, walkers=W, precision=64, seed=5)
@@ -71,11 +71,11 @@ def test_o_rows_match_central_differences(tmp_path, name, over):
     eng.close()
 
 
-@pytest.mark.parametrize("measure", ["packed", "l2"])
+@pytest.mark.parametrize("measure", ["tiles", "l2"])
 def test_o_rows_match_oracle_sroopt_on_32_walkers(tmp_path, monkeypatch, measure):
     """2D 16x16 (t' = -0.2, 112 + 112 electrons, n = 224): every configuration of the 32
-    chains equals the oracle's, and so do the SROptO rows — with the planes swept as packed
-    triangles in shared memory (default) and in place in L2."""
+    chains equals the oracle's, and so do the SROptO rows — with the planes swept as tiles in
+    shared memory (default) and in place in L2."""
     if measure == "l2":
         monkeypatch.setenv("MVMC_B200_MEASURE", "l2")
     else:
@@ -99,7 +99,7 @@ def test_o_rows_match_oracle_sroopt_on_32_walkers(tmp_path, monkeypatch, measure
 def test_o_rows_are_bitwise_repeatable(tmp_path, name):
     """The same saved samples measured twice give bit-identical O rows, energies and sums:
     every reduction, the Slater derivative included, runs in a fixed order (2D 8x8 with 8
-    QP planes in shared memory; 2D 16x16, n = 224, packed triangles)."""
+    QP planes and 2D 16x16, n = 224, both on tiles)."""
     nl, init, dims = inputs(tmp_path, name, 1)
     eng = mvmc().Engine(nl, init, walkers=64, precision=64, seed=3)
     eng.sample()

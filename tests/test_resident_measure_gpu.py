@@ -13,8 +13,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("name,over,guard,rtol", [
     ("chain16", {}, 0.0, 1e-9),                     # n = 16, planes in shared memory
-    ("square16", {"samples": 2}, 0.0, 1e-9),        # n = 224, one plane, packed measurement
-    ("square8", {"interval": 4}, 1e-3, 1e-5),       # eight QP planes in L2, refresh guard on
+    ("square16", {"samples": 2}, 0.0, 1e-9),        # n = 224, one plane, tile measurement
+    ("square8", {"interval": 4}, 1e-3, 1e-5),       # eight QP planes, refresh guard on
 ])
 def test_resident_measurement_matches_recomputed(tmp_path, name, over, guard, rtol):
     """Energies and O rows within rtol relative of the recomputed measurement: the inverse
